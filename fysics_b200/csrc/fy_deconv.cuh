@@ -14,10 +14,13 @@
 // Algorithmic traffic at p = n (no padding): P1 4+4 (1+4 from u8), P2 8, P3 8, P4 8,
 // P5 4+4 bytes per voxel.
 //
-// Kernels take N > 0 for a compile-time FFT plan of length N on their axis (instantiated
-// for the common padded sizes in fy_deconv_ct_*.cu, compiled in parallel), or N = 0 for the
-// runtime plan (fy_deconv.cu). fy_deconv_pass<N> enqueues one of the five passes.
+// fy_deconv_pass<N> enqueues one of the five passes; the units fy_deconv_ct_*.cu, compiled in
+// parallel, instantiate it for the common padded sizes. Axis lengths with a register plan
+// (rf::served: 64 ... 512) run the kernels of fy_regpass.cuh. The kernels here serve the others:
+// N > 0 is a compile-time plan of length N in shared memory (768, 1024), N = 0 the runtime plan
+// (fy_deconv.cu).
 #include "fy_internal.h"
+#include "fy_regpass.cuh"
 
 namespace {
 // Line transform with a compile-time plan when N > 0 (n == N, pitch PS), else the
@@ -51,31 +54,6 @@ FY_D void fft_line_pre(float2* __restrict__ sline, int ps, int tl, const FftPlan
 }
 // Threads per CTA never exceed W*n/E: 512 for 2^k lines (E=16), 256 for 3*2^k (E=24).
 template <int E> struct KB { static constexpr int nt = (E % 3 == 0) ? 256 : 512; };
-// Lines per tile of a column pass with a compile-time length N: the FFT core's tile
-// (ct_tile_lines; N = 0: the runtime plan's, fy_tile_shape), or with NARROW 8 lines of 512
-// points (256 threads, four CTAs per SM), so one CTA's loads overlap three others' transforms.
-// Measured at 512^3: the forward Y pass 266 -> 253 us narrow; the inverse Y pass unchanged;
-// the Z pass 426 -> 466 us (its transform pair per tile keeps the SM busy either way).
-template <int N, int E, bool NARROW> struct YZ {
-    static constexpr bool on = NARROW && N == 512;
-    static constexpr int lines = on ? 8 : ct_pitch(N);
-    static constexpr int nt = on ? 256 : KB<E>::nt;
-    static constexpr int minb = on ? 4 : 2;
-};
-template <int N, bool NARROW> TileShape yz_tile_shape(int n) {
-    if constexpr (YZ<N, 16, NARROW>::on) {
-        TileShape t;
-        t.W = YZ<N, 16, NARROW>::lines;
-        t.wlog = fy_log2i(t.W);
-        t.E = 16;
-        t.NT = t.W * N / t.E;
-        return t;
-    } else {
-        return fy_tile_shape(n);
-    }
-}
-
-
 // Thread -> (line l, thread-in-line tl) with the line index fastest.
 struct Lane {
     int l, tl;
@@ -253,7 +231,7 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_x_fwd(const T* __restrict__ sr
 // straight from global memory (W consecutive columns = one 8W-byte run per point);
 // rows >= ny are the reflected (or zero) rows.
 template <int N, int E>
-__global__ void __launch_bounds__(YZ<N, E, true>::nt, YZ<N, E, true>::minb) k_y_fwd(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ FftPlan pl,
+__global__ void __launch_bounds__(KB<E>::nt, 2) k_y_fwd(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ FftPlan pl,
                                                  const float2* __restrict__ tw, int wlog) {
     fy_pdl_wait();
     extern __shared__ float4 smem4[];
@@ -262,7 +240,7 @@ __global__ void __launch_bounds__(YZ<N, E, true>::nt, YZ<N, E, true>::minb) k_y_
     float2* stw = s + pl.n * W;
     const Lane ln(wlog);
     float2* col = spec + (size_t)blockIdx.y * g.py * g.hxp + blockIdx.x * W + ln.l;
-    fft_line_pre<N, E, YZ<N, E, true>::lines, -1>(s + ln.l, W, ln.tl, pl, stw,
+    fft_line_pre<N, E, ct_pitch(N), -1>(s + ln.l, W, ln.tl, pl, stw,
                 [&](int i) {
                     const int ys = i < g.ny ? i : (g.zero_pad ? -1 : reflect_idx(i, g.ny));
                     return ys < 0 ? make_float2(0.f, 0.f) : col[(size_t)ys * g.hxp];
@@ -422,6 +400,8 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_x_inv(const float2* __restrict
 // length) or the runtime plans (N = 0).
 template <int N>
 cudaError_t fy_deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
+    if constexpr (rf::served(N)) return rf::deconv_pass<N>(pass, d, st);
+    else {
     const SpecGeom& g = d.g;
     const long Q = (long)g.nz * g.ny;
     auto with_e = [&](int n, auto&& body) -> cudaError_t {
@@ -455,7 +435,7 @@ cudaError_t fy_deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
     }
     case 2:     // Y forward over the stored planes
     case 4: {   // Y inverse, keep rows < ny
-        const TileShape t = pass == 2 ? yz_tile_shape<N, true>(g.py) : yz_tile_shape<N, false>(g.py);
+        const TileShape t = fy_tile_shape(g.py);
         const size_t smem = (size_t)g.py * t.W * sizeof(float2) + (size_t)g.py * sizeof(float2);
         dim3 grid(ceil_div_i(g.hx, t.W), g.nz);
         return with_e(g.py, [&](auto ec) -> cudaError_t {
@@ -521,6 +501,7 @@ cudaError_t fy_deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
     }
     default:
         return cudaErrorInvalidValue;
+    }
     }
 }
 

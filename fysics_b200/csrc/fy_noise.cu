@@ -7,12 +7,12 @@
 //      voxels use v = S2'/wc - (S1'/wc)^2, which equals the reference's S2/wc - (S1/wc)^2
 //      without its cancellation.
 //   2. Exact order statistics on orderable 32-bit float keys: the 1st and 99th percentiles
-//      of m (noise.c:104-108) through a sample-guided window, one pass over m and a radix
-//      select of the window's candidates (falling back to radix passes over m when the
-//      window misses), and, per intensity bin with >= 200 voxels, the flat_pct percentile of
-//      v (noise.c:117-134) through the same scheme over mean and variance (falling back to
-//      radix passes over v); each interpolated between order statistics k and k+1 exactly
-//      as percentile() does (noise.c:66-73).
+//      of m (noise.c:104-108) and, per intensity bin with >= 200 voxels, the flat_pct percentile
+//      of v (noise.c:117-134), each interpolated between order statistics k and k+1 exactly as
+//      percentile() does (noise.c:66-73). Each of the two selections reads its fields once, through
+//      sample-guided windows (section 2w): sample and bounds, count, bucket, collect. Radix passes
+//      over the window's candidates or over the whole field stand behind them (section 2r) and
+//      exit at once when the windows gave the answer.
 //   3. k_noise_fit: one thread, FP64: IRLS line fit var = g*I + b (noise.c:137-172) and
 //      noise_ref = sqrt(max(g*ref + b, ..))*1.15 (noise.c:181-187), plus the guided eps
 //      (3*noise_ref)^2 floored at 1e-8 (noise.c:197-202).
@@ -27,14 +27,12 @@
 namespace {
 
 constexpr int NB = 24;                 // intensity bins, noise.c:111
-constexpr int NT_MAX = 64;             // selection targets: 2 per bin + spare
-// ctl->mode: 0 mean percentiles by radix passes, 1 bin percentiles by radix passes, 2
-// variance fallback, 3 done; kModeWin0: the mean percentiles through the sample-guided
-// window (section 2w), which falls back to mode 0 when the window misses.
-constexpr int kModeWin0 = 4;
-constexpr int kModeBinCand = 6;        // the bins' last digit runs on a candidate list (cc)
-constexpr int kModeBinWin = 7;         // the bins' percentiles through the sample-guided window (2bw)
-constexpr int kModeBinDone = 8;        // the window found them: the bins' radix passes stand aside
+// ctl->mode: which step acts next. The window steps of the means (kMeanWin) and of the bins
+// (kBinWin) hand over to their radix passes: over the candidates (kMeanCand, kBinCand) when one
+// bucket holds too many keys to collect, over the whole field (kMeanField, kBinField) when a
+// window missed or its candidate list overflowed. kVarField: no bin qualifies, the percentile of
+// all variances (noise.c:166-171).
+enum { kMeanWin, kMeanCand, kMeanField, kBinWin, kBinCand, kBinField, kVarField };
 
 FY_D uint32_t fkey(float f) {
     const uint32_t u = __float_as_uint(f);
@@ -55,44 +53,44 @@ FY_HD float funkey(uint32_t k) {
 }  // namespace
 
 // Device-resident control block of one estimate (lives in the caller's scratch).
-// Selection targets: target t selects the order statistic k_t (0-based) of the keys of
-// group g_t. Bins: t = bin id. Whole volume: t = 0, 1 (1st/99th percentile) or t = 0
-// (variance fallback). After the digit passes, prefix_t is the k-th key, eq_t the number of
-// keys equal to it and rank_t its rank among them; the (k+1)-th key is the same key when
-// rank_t + 1 < eq_t, else the smallest key greater than it (k_sel_next).
+// Selection targets: target t selects the order statistic k_t (0-based) of the keys of its
+// group: the 1st/99th percentile (t = 0, 1), a bin (t = bin), or all variances (t = 0). When a
+// selection has ended, prefix_t is the k-th key, and the (k+1)-th is the same key unless
+// tneed_next, then tnext.
+constexpr int kHist = NB * 256;        // the targets' histograms: 256 digits each, or window buckets
 struct NoiseCtl {
     long long n;
     double flat_pct, ref_intensity;
-    int ntarget, mode;                 // mode 0 means lo/hi, 1 bins, 2 variance fallback, 3 done
-    long long tk[NT_MAX];              // requested rank k
-    long long trank[NT_MAX];           // remaining rank inside the decided prefix
-    long long tgroup_n[NT_MAX];        // group size
-    unsigned long long teq[NT_MAX];    // keys equal to the selected key
-    uint32_t tprefix[NT_MAX];
-    uint32_t tnext[NT_MAX];            // min key > selected key (when needed)
-    int tactive[NT_MAX];
-    int tneed_next[NT_MAX];
-    double lo, hi;
+    int ntarget, mode;
+    long long tk[NB];                  // requested rank k
+    long long trank[NB];               // remaining rank inside the decided prefix
+    long long tgroup_n[NB];            // group size
+    unsigned long long teq[NB];        // keys equal to the selected key
+    uint32_t tprefix[NB];
+    uint32_t tnext[NB];                // smallest key above the selected one (when needed)
+    uint32_t tabove[NB];               // radix passes: smallest key above the last digit's prefix
+    int tactive[NB];
+    int tneed_next[NB];
     double edge[NB + 1];
     float fedge[NB + 1];               // smallest float >= edge[k]: exact float membership test
-    float fscale;                      // NB/(hi-lo) for the bin guess
     unsigned long long bcount[NB];
-    double bfloor[NB];
     double out_g, out_b, out_noise_ref, out_ref_intensity;
     int out_used;
     float eps;                         // fy_guided_eps_for_noise(noise_ref), for a chained guided filter
-    alignas(16) unsigned int hist[NT_MAX * 256];   // per-target histogram (bins: 24 x 256; whole: 2 x 2048)
-    // Sample-guided window (section 2w): per target the window keys [wlo, whi] and the count
-    // of keys below wlo.
-    uint32_t wlo[2], whi[2];
-    unsigned long long wbelow[2];
+    alignas(16) unsigned int hist[kHist];
+    // windows (section 2w): per target the keys [wlo, whi], the group's keys below wlo and, for a
+    // bin, its voxels; the candidate list's length; the bucket origin and scale of the window's
+    // values; the buckets that hold the ranks k and k+1, the rank within them and the keys collected
+    uint32_t wlo[NB], whi[NB];
+    uint32_t klo[NB], khi[NB];         // the sample's keys that bound the window (its ends, where it has some)
+    unsigned long long wbelow[NB], wvox[NB];
     unsigned long long ncand;          // candidates appended (may exceed the capacity)
-    int wfail;                         // the window missed: the radix passes run instead
-    // The bins' windows (section 2bw): per bin the variance keys [bwlo, bwhi] and the counts
-    // of the bin's keys below, inside and above it.
-    uint32_t bwlo[NB], bwhi[NB];
-    unsigned long long bwc[NB * 3];
-    unsigned int done_ctas;            // CTAs of the current digit pass that have flushed (0 between passes)
+    float cv0[NB], cvs[NB];
+    int cb0[NB], cb1[NB];
+    long long crank[NB];
+    unsigned int ccnt[NB];
+    unsigned int bsn[NB];              // sample keys listed per bin (may exceed the list's capacity)
+    unsigned int done_ctas;            // CTAs of the current step that have finished (0 between steps)
 };
 
 namespace {
@@ -108,7 +106,32 @@ FY_D unsigned vgx() { return s_vgx; }
 // ---------------------------------------------------------------- 1. local stats
 // z-sliding box pass (fy_zbox.cuh, ZB_NOISE): 4 B read + 8 B written per voxel.
 
-// ---------------------------------------------------------------- 2. radix select
+// The CTA of the volume that gets here last (a ticket) returns true, with every other CTA's
+// writes before its own ticket visible; it then sets done_ctas back to 0.
+FY_D bool last_cta(NoiseCtl* ctl) {
+    __shared__ int s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&ctl->done_ctas, 1u) == vgx() - 1;
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+    return true;
+}
+
+FY_D void target_init(NoiseCtl* ctl, int t, long long k, long long group_n, bool on) {
+    ctl->tk[t] = k;
+    ctl->trank[t] = k;
+    ctl->tgroup_n[t] = group_n;
+    ctl->tprefix[t] = 0;
+    ctl->teq[t] = 0;
+    ctl->tactive[t] = on;
+    ctl->tneed_next[t] = 0;
+    ctl->tnext[t] = 0xffffffffu;
+    ctl->tabove[t] = 0xffffffffu;
+}
+
+// ---------------------------------------------------------------- 2r. radix select
 // Exact bin of a float mean: m >= edge[k] <=> m >= fedge[k] with fedge[k] the smallest float
 // >= edge[k] (noise.c:118-122 in double), so membership needs only float compares.
 FY_D int bin_of(float m, const float* __restrict__ fe, float lo_f, float scale) {
@@ -117,19 +140,6 @@ FY_D int bin_of(float m, const float* __restrict__ fe, float lo_f, float scale) 
     b = b < 0 ? 0 : (b > NB - 1 ? NB - 1 : b);
     while (b > 0 && m < fe[b]) --b;
     while (b < NB - 1 && m >= fe[b + 1]) ++b;
-    return b;
-}
-
-// bin_of with at most one step from the float guess (the guess is within one bin of the
-// exact one unless the range [lo, hi] is degenerate; then the exact walk runs): the common
-// path has no loop. lo_e, hi_e: fe[0], fe[NB].
-FY_D int bin_fast(float m, const float* __restrict__ fe, float lo_e, float hi_e, float lo_f, float scale) {
-    if (!(m >= lo_e && m < hi_e)) return -1;
-    int b = (int)((m - lo_f) * scale);
-    b = b < 0 ? 0 : (b > NB - 1 ? NB - 1 : b);
-    b -= (int)(m < fe[b]);                      // m >= fe[0], so b stays >= 0
-    b += (int)(m >= fe[b + 1]);                 // m < fe[NB], so b stays <= NB - 1
-    if (m < fe[b] || m >= fe[b + 1]) b = bin_of(m, fe, lo_f, scale);
     return b;
 }
 
@@ -155,9 +165,8 @@ struct RunAcc {
     }
 };
 
-constexpr int kWarpBuf = 256;
 struct WarpCands {
-    float* v;                          // this warp's kWarpBuf values in shared memory
+    float* v;                          // this warp's values in shared memory
     uint8_t* l;                        // and labels
     int cnt = 0;                       // warp-uniform fill
     FY_D void flush(float* __restrict__ cval, uint8_t* __restrict__ clab, unsigned long long* ncand, long long cap) {
@@ -180,50 +189,25 @@ struct WarpCands {
 // loop run without per-element range checks; the one partial chunk is checked.
 constexpr int SU = 4;
 
-// One digit pass (bits [shift, shift + DB)) for every active target whose prefix matches.
-// MODE 0: keys of mean, targets 0 and 1 over all voxels; MODE 1: keys of var, target = bin;
-// MODE 2: keys of var, target 0 over all voxels. A key matches at most one distinct prefix,
-// so in modes 0/2 targets whose prefixes are equal share one shared-memory histogram
-// (group) and every voxel makes at most one increment; the flush copies a group's counts
-// to each of its targets. Inactive targets and bin label 255 carry the prefix 0xffffffff,
-// which no key's high part (< 2^(32 - shift - DB)) can equal.
-// LABEL (the first variance pass only): the bin of each voxel is computed from its mean here
-// and its u8 label written for the later passes, so no separate labelling pass runs.
-// COMPACT (a MODE 1 digit pass): each voxel whose key matches its bin target's prefix is also
-// appended, with its bin, to the candidate list (cval, clab; counter ctl->ncand): every key of
-// the prefixes that the following digits narrow is then in the list.
-// scan >= 0: the CTA that flushes last (a ticket on ctl->done_ctas) then does every active
-// target's bookkeeping (warp_scan_target; scan 1: after the last digit), so no separate scan
-// launch follows the pass.
-constexpr int kCompactBuf = 1152;        // per warp: one step's worst case (32 x 4*SU) + slack
-
 // The bookkeeping after a digit pass for target t, by one warp: the bucket that holds the
 // target's rank (a warp scan of the lanes' bucket sums), the prefix extended by it, the keys
-// equal to the selected key and, after the last digit, the next non-empty bucket (the
-// smallest key above the selected one within the prefix; k_sel_next scans only when there is
-// none). The histogram is read through L2 (other CTAs' atomics) and cleared.
-// With at most 8 buckets per lane (8-bit digits) the lane's buckets stay in registers: one
-// round of loads (with the target's rank and prefix) instead of one per reading.
-template <int DB>
+// equal to the selected key and, after the last digit, the smallest key above the selected one:
+// the next non-empty bucket within the prefix, else the smallest key above the prefix, which
+// the last pass recorded. The histogram is read through L2 (other CTAs' atomics) and cleared.
 FY_D void warp_scan_target(NoiseCtl* ctl, int t, bool last) {
-    constexpr int nbk = 1 << DB, per = nbk / 32;
-    constexpr bool REG = per <= 8;
+    constexpr int per = 256 / 32;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    unsigned int* h = ctl->hist + (size_t)t * nbk;
+    unsigned int* h = ctl->hist + t * 256;
     const int b0 = lane * per;
     const long long r = ctl->trank[t];
     const uint32_t pre = ctl->tprefix[t];
-    unsigned int hv[REG ? per : 1];
+    unsigned int hv[per];
     unsigned long long mine = 0;
-    if (REG) {
 #pragma unroll
-        for (int i = 0; i < (REG ? per : 1); ++i) hv[i] = __ldcg(h + b0 + i);
+    for (int i = 0; i < per; ++i) hv[i] = __ldcg(h + b0 + i);
 #pragma unroll
-        for (int i = 0; i < (REG ? per : 1); ++i) mine += hv[i];
-    } else {
-        for (int b = b0; b < b0 + per; ++b) mine += __ldcg(h + b);
-    }
+    for (int i = 0; i < per; ++i) mine += hv[i];
     unsigned long long incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -231,162 +215,112 @@ FY_D void warp_scan_target(NoiseCtl* ctl, int t, bool last) {
         if (lane >= o) incl += y;
     }
     const unsigned long long before = incl - mine;
-    unsigned int sel = (unsigned)nbk;
+    unsigned int sel = 256;
     if ((unsigned long long)r >= before && (unsigned long long)r < incl) {
         unsigned long long acc = before;
         unsigned int hsel = 0;
-        if (REG) {
 #pragma unroll
-            for (int i = 0; i < (REG ? per : 1); ++i) {
-                if (sel == (unsigned)nbk && acc + hv[i] > (unsigned long long)r) { sel = (unsigned)(b0 + i); hsel = hv[i]; }
-                else if (sel == (unsigned)nbk) acc += hv[i];
-            }
-        } else {
-            for (int b = b0; b < b0 + per; ++b) {
-                const unsigned int hb = __ldcg(h + b);
-                if (acc + hb > (unsigned long long)r) { sel = (unsigned)b; hsel = hb; break; }
-                acc += hb;
-            }
+        for (int i = 0; i < per; ++i) {
+            if (sel == 256 && acc + hv[i] > (unsigned long long)r) { sel = (unsigned)(b0 + i); hsel = hv[i]; }
+            else if (sel == 256) acc += hv[i];
         }
-        if (sel != (unsigned)nbk) {
-            ctl->trank[t] = r - (long long)acc;
-            ctl->tprefix[t] = (pre << DB) | sel;
-            if (last) ctl->teq[t] = hsel;
-        }
+        ctl->trank[t] = r - (long long)acc;
+        ctl->tprefix[t] = (pre << 8) | sel;
+        if (last) ctl->teq[t] = hsel;
     }
     sel = __reduce_min_sync(full, sel);
     unsigned int nextb = 0xffffffffu;
     if (last) {
-        if (REG) {
 #pragma unroll
-            for (int i = (REG ? per : 1) - 1; i >= 0; --i)
-                if (b0 + i > (int)sel && hv[i]) nextb = (unsigned)(b0 + i);
-        } else {
-            for (int b = b0 > (int)sel + 1 ? b0 : (int)sel + 1; b < b0 + per; ++b)
-                if (__ldcg(h + b)) { nextb = (unsigned)b; break; }
-        }
+        for (int i = per - 1; i >= 0; --i)
+            if (b0 + i > (int)sel && hv[i]) nextb = (unsigned)(b0 + i);
         nextb = __reduce_min_sync(full, nextb);
     }
     __syncwarp();
-    for (int b = b0; b < b0 + per; ++b) h[b] = 0;
+#pragma unroll
+    for (int i = 0; i < per; ++i) h[b0 + i] = 0;
     __syncwarp();
     if (last && lane == 0) {
         ctl->tneed_next[t] = (ctl->trank[t] + 1 >= (long long)ctl->teq[t]) && (ctl->tk[t] + 1 < ctl->tgroup_n[t]);
-        ctl->tnext[t] = nextb != 0xffffffffu ? ((ctl->tprefix[t] >> DB) << DB) | nextb : 0xffffffffu;
+        ctl->tnext[t] = nextb != 0xffffffffu ? (pre << 8) | nextb : __ldcg(&ctl->tabove[t]);
     }
 }
-template <int DB, int MODE, bool LABEL = false, bool COMPACT = false>
-FY_D void k_sel_hist(const float* __restrict__ mean, const float* __restrict__ var,
-                                                  uint8_t* __restrict__ bin, NoiseCtl* __restrict__ ctl,
-                                                  int shift, float* __restrict__ cval = nullptr,
-                                                  uint8_t* __restrict__ clab = nullptr, long long cap = 0,
-                                                  int scan = -1) {
-    fy_pdl_wait();
-    extern __shared__ unsigned int h[];
+
+// One 8-bit digit pass (bits [shift, shift + 8)) over n keys for every active target whose prefix
+// matches. LAB 0: no labels, every key belongs to every target (at most two; targets whose
+// prefixes are equal share one shared-memory histogram, so a key makes at most one increment, and
+// the flush copies a group's counts to each of its targets). LAB 1: the key's target is its u8
+// label. LAB 2 (the first pass over the bins): the label is computed from the voxel's mean and
+// written for the later passes. Inactive targets and label 255 carry the prefix 0xffffffff, which
+// no key's high part can equal. The last pass also records, per target, the smallest key above
+// the prefix.
+template <int LAB>
+FY_D void radix_pass(const float* __restrict__ src, const float* __restrict__ mean, uint8_t* __restrict__ lab8,
+                     long long n, NoiseCtl* __restrict__ ctl, int shift, unsigned int* __restrict__ h) {
     __shared__ uint32_t sp[256];
+    __shared__ unsigned int smin[NB];
     __shared__ float fe[NB + 1];
-    if (ctl->mode != MODE) return;
-    if (LABEL && threadIdx.x <= NB) fe[threadIdx.x] = ctl->fedge[threadIdx.x];
-    const float lo_f = LABEL ? ctl->fedge[0] : 0.f, fscale = LABEL ? ctl->fscale : 0.f;
-    auto lab = [&](float m) -> unsigned { const int b = bin_of(m, fe, lo_f, fscale); return b < 0 ? 255u : (unsigned)b; };
-    constexpr int NBK = 1 << DB;
-    const int nt = ctl->ntarget;
-    if (MODE == 1)
-        for (int i = threadIdx.x; i < 256; i += blockDim.x) sp[i] = i < nt && ctl->tactive[i] ? ctl->tprefix[i] : 0xffffffffu;
-    // modes 0/2: at most two targets; group of target 1 is 0 when it shares target 0's prefix
+    const int nt = ctl->ntarget, top = shift + 8;
+    if (LAB == 2 && threadIdx.x <= NB) fe[threadIdx.x] = ctl->fedge[threadIdx.x];
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) sp[i] = i < nt && ctl->tactive[i] ? ctl->tprefix[i] : 0xffffffffu;
+    if (threadIdx.x < NB) smin[threadIdx.x] = 0xffffffffu;
     uint32_t p0 = 0xffffffffu, p1 = 0xffffffffu;
-    int g1 = 1;
-    if (MODE != 1) {
-        p0 = ctl->tactive[0] ? ctl->tprefix[0] : 0xffffffffu;
+    int g1 = 1;                                          // target 1's histogram: 0 when it shares target 0's prefix
+    if (LAB == 0) {
+        if (ctl->tactive[0]) p0 = ctl->tprefix[0];
         if (nt > 1 && ctl->tactive[1]) {
             p1 = ctl->tprefix[1];
-            if (p1 == p0) { g1 = 0; p1 = 0xfffffffeu; }   // never matches: target 1 reads group 0
+            if (p1 == p0) { g1 = 0; p1 = 0xfffffffeu; }  // never matches
         }
     }
-    const int ngroup = MODE == 1 ? nt : 2;
-    for (int i = threadIdx.x; i < ngroup * NBK; i += blockDim.x) h[i] = 0;
+    for (int i = threadIdx.x; i < (LAB == 0 ? 2 : nt) * 256; i += blockDim.x) h[i] = 0;
     __syncthreads();
-    const int top = shift + DB;
-    const long long n = ctl->n, n4 = (n + 3) / 4, n4f = n / 4;
-    const float* src = MODE == 0 ? mean : var;
-    const int step = blockDim.x;
-    const long long chunk = (long long)SU * step;
+    const float lo_f = LAB == 2 ? fe[0] : 0.f, fscale = LAB == 2 ? (float)(NB / (ctl->edge[NB] - ctl->edge[0])) : 0.f;
+    auto label = [&](float m) -> unsigned { const int b = bin_of(m, fe, lo_f, fscale); return b < 0 ? 255u : (unsigned)b; };
     RunAcc acc;
-    auto code_of = [&](float v, int g) -> int {
+    uint32_t a0 = 0xffffffffu, a1 = 0xffffffffu;          // LAB 0: smallest key above the prefix of targets 0, 1
+    const uint32_t q1 = g1 ? p1 : p0;
+    auto visit = [&](float v, unsigned g) {
         const uint32_t key = fkey(v);
         const uint32_t hb = top >= 32 ? 0u : (key >> top);
-        const int dig = (key >> shift) & (NBK - 1);
-        if (MODE == 1) return sp[g] == hb ? g * NBK + dig : -1;
-        return hb == p0 ? dig : (hb == p1 ? NBK + dig : -1);
+        const int dig = (key >> shift) & 255;
+        if (LAB) {
+            const uint32_t pg = sp[g];
+            acc.add(h, pg == hb ? (int)g * 256 + dig : -1);
+            if (shift == 0 && hb > pg && key < smin[g]) atomicMin(&smin[g], key);
+        } else {
+            acc.add(h, hb == p0 ? dig : (hb == p1 ? 256 + dig : -1));
+            if (shift == 0) {
+                if (hb > p0) a0 = min(a0, key);
+                if (hb > q1) a1 = min(a1, key);
+            }
+        }
     };
-    WarpCands wc;
-    if (COMPACT) {
-        float* bv = reinterpret_cast<float*>(h + ngroup * NBK);
-        wc.v = bv + (threadIdx.x >> 5) * kCompactBuf;
-        wc.l = reinterpret_cast<uint8_t*>(bv + (blockDim.x >> 5) * kCompactBuf) + (threadIdx.x >> 5) * kCompactBuf;
-    }
+    const int step = blockDim.x;
+    const long long n4 = (n + 3) / 4, n4f = n / 4, chunk = (long long)SU * step;
     long long base = (long long)vbx() * chunk;
     const long long stride = (long long)vgx() * chunk;        // read once: the loop body has syncs
     for (; base + chunk <= n4f; base += stride) {
         float4 x[SU];
         uchar4 bb[SU];
-        float4 mm[LABEL ? SU : 1];
+        float4 mm[LAB == 2 ? SU : 1];
 #pragma unroll
         for (int u = 0; u < SU; ++u) {
             const long long q = base + threadIdx.x + (long long)u * step;
             x[u] = __ldg(reinterpret_cast<const float4*>(src) + q);
-            if (LABEL) mm[u] = __ldg(reinterpret_cast<const float4*>(mean) + q);
-            else if (MODE == 1) bb[u] = __ldg(reinterpret_cast<const uchar4*>(bin) + q);
+            if (LAB == 2) mm[u] = __ldg(reinterpret_cast<const float4*>(mean) + q);
+            else if (LAB) bb[u] = *(reinterpret_cast<const uchar4*>(lab8) + q);
         }
-        if (LABEL) {
 #pragma unroll
-            for (int u = 0; u < SU; ++u) {
-                bb[u] = make_uchar4(lab(mm[u].x), lab(mm[u].y), lab(mm[u].z), lab(mm[u].w));
-                reinterpret_cast<uchar4*>(bin)[base + threadIdx.x + (long long)u * step] = bb[u];
+        for (int u = 0; u < SU; ++u) {
+            if (LAB == 2) {
+                bb[u] = make_uchar4(label(mm[u].x), label(mm[u].y), label(mm[u].z), label(mm[u].w));
+                reinterpret_cast<uchar4*>(lab8)[base + threadIdx.x + (long long)u * step] = bb[u];
             }
-        }
-        if (!COMPACT) {
-#pragma unroll
-            for (int u = 0; u < SU; ++u) {
-                acc.add(h, code_of(x[u].x, MODE == 1 ? bb[u].x : 0));
-                acc.add(h, code_of(x[u].y, MODE == 1 ? bb[u].y : 0));
-                acc.add(h, code_of(x[u].z, MODE == 1 ? bb[u].z : 0));
-                acc.add(h, code_of(x[u].w, MODE == 1 ? bb[u].w : 0));
-            }
-        } else {
-            float xv[4 * SU];
-            unsigned xl[4 * SU];
-            unsigned hit = 0;
-#pragma unroll
-            for (int u = 0; u < SU; ++u) {
-                xv[4 * u] = x[u].x; xv[4 * u + 1] = x[u].y; xv[4 * u + 2] = x[u].z; xv[4 * u + 3] = x[u].w;
-                xl[4 * u] = bb[u].x; xl[4 * u + 1] = bb[u].y; xl[4 * u + 2] = bb[u].z; xl[4 * u + 3] = bb[u].w;
-            }
-#pragma unroll
-            for (int q = 0; q < 4 * SU; ++q) {
-                const int code = code_of(xv[q], (int)xl[q]);
-                acc.add(h, code);
-                hit |= (unsigned)(code >= 0) << q;
-            }
-            // place this step's hits in the warp's buffer (one scan), append it when nearly full
-            const unsigned full = 0xffffffffu;
-            const int lane = threadIdx.x & 31, c = __popc(hit);
-            int incl = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(full, incl, o);
-                if (lane >= o) incl += y;
-            }
-            const int tot = __shfl_sync(full, incl, 31);
-            if (tot) {
-                if (wc.cnt + tot > kCompactBuf) wc.flush(cval, clab, &ctl->ncand, cap);
-                int pos = wc.cnt + incl - c;
-#pragma unroll
-                for (int q = 0; q < 4 * SU; ++q)
-                    if ((hit >> q) & 1u) { wc.v[pos] = xv[q]; wc.l[pos] = (uint8_t)xl[q]; ++pos; }
-                wc.cnt += tot;
-                __syncwarp();
-            }
+            visit(x[u].x, LAB ? bb[u].x : 0);
+            visit(x[u].y, LAB ? bb[u].y : 0);
+            visit(x[u].z, LAB ? bb[u].z : 0);
+            visit(x[u].w, LAB ? bb[u].w : 0);
         }
     }
     if (base < n4) {                                     // the grid's partial chunk
@@ -394,162 +328,51 @@ FY_D void k_sel_hist(const float* __restrict__ mean, const float* __restrict__ v
             for (int j = 0; j < 4; ++j) {
                 const long long i = 4 * (base + threadIdx.x + (long long)u * step) + j;
                 if (i >= n) continue;
-                int g = 0;
-                if (LABEL) { g = (int)lab(__ldg(mean + i)); bin[i] = (uint8_t)g; }
-                else if (MODE == 1) g = (int)__ldg(bin + i);
-                const float v = __ldg(src + i);
-                const int code = code_of(v, g);
-                acc.add(h, code);
-                if (COMPACT && code >= 0) {
-                    const unsigned long long pos = atomicAdd(&ctl->ncand, 1ull);
-                    if ((long long)pos < cap) { cval[pos] = v; clab[pos] = (uint8_t)g; }
-                }
+                unsigned g = 0;
+                if (LAB == 2) { g = label(__ldg(mean + i)); lab8[i] = (uint8_t)g; }
+                else if (LAB) g = lab8[i];
+                visit(__ldg(src + i), g);
             }
     }
-    if (COMPACT) wc.flush(cval, clab, &ctl->ncand, cap);
     acc.flush(h);
-    __syncthreads();
-    if (MODE == 1) {
-        for (int i = threadIdx.x; i < nt * NBK; i += blockDim.x)
-            if (h[i]) atomicAdd(&ctl->hist[i], h[i]);
-    } else {
-        for (int i = threadIdx.x; i < nt * NBK; i += blockDim.x) {
-            const int t = i / NBK, grp = t == 0 ? 0 : g1;
-            const unsigned int cnt = h[grp * NBK + (i - t * NBK)];
-            if (cnt) atomicAdd(&ctl->hist[i], cnt);
-        }
+    if (LAB == 0 && shift == 0) {
+        if (a0 != 0xffffffffu) atomicMin(&smin[0], a0);
+        if (a1 != 0xffffffffu) atomicMin(&smin[1], a1);
     }
-    if (scan < 0) return;
-    __shared__ int s_last;
-    __threadfence();                                     // this CTA's counts before its ticket
     __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&ctl->done_ctas, 1u) == vgx() - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
+    for (int i = threadIdx.x; i < nt * 256; i += blockDim.x) {
+        const int t = i >> 8;
+        const unsigned int cnt = h[LAB ? i : (t == 0 ? 0 : g1) * 256 + (i & 255)];
+        if (cnt) atomicAdd(&ctl->hist[i], cnt);
+    }
+    if (shift == 0 && threadIdx.x < nt && smin[threadIdx.x] != 0xffffffffu)
+        atomicMin(&ctl->tabove[threadIdx.x], smin[threadIdx.x]);
+    if (!last_cta(ctl)) return;
     for (int t = threadIdx.x >> 5; t < nt; t += blockDim.x >> 5)
-        if (ctl->tactive[t]) warp_scan_target<DB>(ctl, t, scan == 1);
+        if (ctl->tactive[t]) warp_scan_target(ctl, t, shift == 0);
     if (threadIdx.x == 0) ctl->done_ctas = 0;
 }
 
-// After a digit pass: target t (one block) finds the bucket holding its rank by a block
-// scan of the histogram, extends its prefix, records how many keys share the final key.
-// After the last digit, the next non-empty bucket of that digit is the smallest key above
-// the selected one within the prefix; k_sel_next scans only when there is none.
-FY_D void k_sel_scan(NoiseCtl* __restrict__ ctl, int db, int want_mode, int last) {
+// The radix passes behind the means' windows, and behind the bins': which keys a pass reads
+// follows from ctl->mode; in the common case none, and the launch ends at once.
+FY_D void k_mean_radix(const float* __restrict__ mean, NoiseCtl* __restrict__ ctl, const float* __restrict__ cval,
+                       uint8_t* __restrict__ clab, int shift) {
     fy_pdl_wait();
-    __shared__ unsigned long long part[256];
-    __shared__ int s_sel;
-    __shared__ unsigned int s_nextb;
-    if (ctl->mode != want_mode) return;
-    const int t = vbx();
-    if (t >= ctl->ntarget || !ctl->tactive[t]) return;
-    const int nbk = 1 << db, per = nbk / 256 > 0 ? nbk / 256 : 1;
-    unsigned int* h = ctl->hist + (size_t)t * nbk;
-    const int b0 = threadIdx.x * per;
-    unsigned long long mine = 0;
-    for (int b = b0; b < b0 + per && b < nbk; ++b) mine += h[b];
-    part[threadIdx.x] = mine;
-    if (threadIdx.x == 0) { s_sel = nbk; s_nextb = 0xffffffffu; }
-    __syncthreads();
-    for (int off = 1; off < 256; off <<= 1) {                // inclusive scan
-        const unsigned long long add = threadIdx.x >= off ? part[threadIdx.x - off] : 0ull;
-        __syncthreads();
-        part[threadIdx.x] += add;
-        __syncthreads();
-    }
-    const long long r = ctl->trank[t];
-    const unsigned long long before = threadIdx.x ? part[threadIdx.x - 1] : 0ull;
-    if ((unsigned long long)r >= before && (unsigned long long)r < part[threadIdx.x]) {
-        unsigned long long acc = before;
-        for (int b = b0; b < b0 + per && b < nbk; ++b) {
-            if (acc + h[b] > (unsigned long long)r) {
-                ctl->trank[t] = r - (long long)acc;
-                ctl->tprefix[t] = (ctl->tprefix[t] << db) | (uint32_t)b;
-                if (last) ctl->teq[t] = h[b];
-                s_sel = b;
-                break;
-            }
-            acc += h[b];
-        }
-    }
-    __syncthreads();
-    if (last) {
-        const int sel = s_sel;
-        for (int b = b0 > sel + 1 ? b0 : sel + 1; b < b0 + per && b < nbk; ++b)
-            if (h[b]) { atomicMin(&s_nextb, (unsigned)b); break; }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nbk; i += blockDim.x) h[i] = 0;
-    if (last && threadIdx.x == 0) {
-        ctl->tneed_next[t] = (ctl->trank[t] + 1 >= (long long)ctl->teq[t]) && (ctl->tk[t] + 1 < ctl->tgroup_n[t]);
-        ctl->tnext[t] = s_nextb != 0xffffffffu ? ((ctl->tprefix[t] >> db) << db) | s_nextb : 0xffffffffu;
-    }
+    extern __shared__ unsigned int rh[];
+    const int mode = ctl->mode;
+    if (mode == kMeanField) radix_pass<0>(mean, nullptr, nullptr, ctl->n, ctl, shift, rh);
+    else if (mode == kMeanCand) radix_pass<1>(cval, nullptr, clab, (long long)ctl->ncand, ctl, shift, rh);
 }
-
-// Smallest key greater than the selected key, for targets whose k+1 lies past it and whose
-// last digit histogram held no larger key (k_sel_scan resolves every other target).
-FY_D void k_sel_next(const float* __restrict__ mean, const float* __restrict__ var,
-                                                  const uint8_t* __restrict__ bin, NoiseCtl* __restrict__ ctl,
-                                                  int want_mode) {
+FY_D void k_bin_radix(const float* __restrict__ mean, const float* __restrict__ var, uint8_t* __restrict__ bin,
+                      NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, uint8_t* __restrict__ clab, int shift) {
     fy_pdl_wait();
-    __shared__ uint32_t sp[NT_MAX];
-    __shared__ int sn[NT_MAX];
-    __shared__ unsigned int smin[NT_MAX];
-    __shared__ int s_any;
-    if (ctl->mode != want_mode) return;
-    const int nt = ctl->ntarget;
-    if (threadIdx.x == 0) s_any = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
-        sp[i] = ctl->tprefix[i];
-        sn[i] = ctl->tactive[i] && ctl->tneed_next[i] && ctl->tnext[i] == 0xffffffffu;
-        smin[i] = 0xffffffffu;
-        if (sn[i]) s_any = 1;
-    }
-    __syncthreads();
-    if (!s_any) return;
-    const long long n = ctl->n;
-    const float* src = want_mode == 0 ? mean : var;
-    auto visit = [&](float v, int g) {
-        const uint32_t key = fkey(v);
-        if (want_mode == 1) {            // one target per voxel: its bin
-            if (g < NB && g < nt && sn[g] && key > sp[g] && key < smin[g]) atomicMin(&smin[g], key);
-        } else {
-            for (int t = 0; t < nt; ++t)
-                if (sn[t] && key > sp[t] && key < smin[t]) atomicMin(&smin[t], key);
-        }
-    };
-    // SU float4 (and uchar4 labels) per thread before any is used, as the streaming passes
-    const long long n4 = (n + 3) / 4, n4f = n / 4, chunk = (long long)SU * blockDim.x;
-    long long base = (long long)vbx() * chunk;
-    const long long stride = (long long)vgx() * chunk;        // read once: the loop body has syncs
-    for (; base + chunk <= n4f; base += stride) {
-        float4 x[SU];
-        uchar4 bb[SU];
-#pragma unroll
-        for (int u = 0; u < SU; ++u) {
-            const long long q = base + threadIdx.x + (long long)u * blockDim.x;
-            x[u] = __ldg(reinterpret_cast<const float4*>(src) + q);
-            bb[u] = want_mode == 1 ? __ldg(reinterpret_cast<const uchar4*>(bin) + q) : make_uchar4(0, 0, 0, 0);
-        }
-#pragma unroll
-        for (int u = 0; u < SU; ++u) {
-            visit(x[u].x, bb[u].x);
-            visit(x[u].y, bb[u].y);
-            visit(x[u].z, bb[u].z);
-            visit(x[u].w, bb[u].w);
-        }
-    }
-    if (base < n4)                                       // the grid's partial chunk
-        for (int u = 0; u < SU; ++u)
-            for (int j = 0; j < 4; ++j) {
-                const long long i = 4 * (base + threadIdx.x + (long long)u * blockDim.x) + j;
-                if (i < n) visit(__ldg(src + i), want_mode == 1 ? (int)__ldg(bin + i) : 0);
-            }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nt; i += blockDim.x)
-        if (sn[i] && smin[i] != 0xffffffffu) atomicMin(&ctl->tnext[i], smin[i]);
+    extern __shared__ unsigned int rh[];
+    const int mode = ctl->mode;
+    if (mode == kBinField) {
+        if (shift == 24) radix_pass<2>(var, mean, bin, ctl->n, ctl, shift, rh);
+        else radix_pass<1>(var, nullptr, bin, ctl->n, ctl, shift, rh);
+    } else if (mode == kBinCand) radix_pass<1>(cval, nullptr, clab, (long long)ctl->ncand, ctl, shift, rh);
+    else if (mode == kVarField) radix_pass<0>(var, nullptr, nullptr, ctl->n, ctl, shift, rh);
 }
 
 // value of order statistic k+1 of target t
@@ -563,260 +386,227 @@ FY_D double interp(const NoiseCtl* ctl, int t, double f, bool has_next) {
     return v0 * (1 - f) + next_value(ctl, t) * f;
 }
 
-FY_D void target_init(NoiseCtl* ctl, int t, long long k, long long group_n, bool on) {
-    ctl->tk[t] = k;
-    ctl->trank[t] = k;
-    ctl->tgroup_n[t] = group_n;
-    ctl->tprefix[t] = 0;
-    ctl->teq[t] = 0;
-    ctl->tactive[t] = on;
-    ctl->tneed_next[t] = 0;
-    ctl->tnext[t] = 0xffffffffu;
-}
-
-// One block of 256 threads: thread t < NT_MAX initialises target t; all clear both blocks'
-// histograms.
-FY_D void k_noise_setup(NoiseCtl* ctl, NoiseCtl* cc, long long n, double flat_pct, double ref_intensity) {
-    fy_pdl_wait();
-    const int t = threadIdx.x;
-    static_assert(sizeof(ctl->hist) % 16 == 0 && offsetof(NoiseCtl, hist) % 16 == 0, "uint4 clears");
-    for (int i = t; i < (int)(sizeof(ctl->hist) / 16); i += blockDim.x) {
-        reinterpret_cast<uint4*>(ctl->hist)[i] = make_uint4(0u, 0u, 0u, 0u);
-        reinterpret_cast<uint4*>(cc->hist)[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
-    if (t >= NT_MAX) return;
-    const double i1 = 1.0 / 100.0 * (double)(n - 1), i99 = 99.0 / 100.0 * (double)(n - 1);
-    if (t == 0) target_init(ctl, 0, (long long)i1, n, true);           // 1st percentile of the means
-    else if (t == 1) target_init(ctl, 1, (long long)i99, n, true);     // 99th
-    else target_init(ctl, t, 0, 0, false);
-    if (t < NB) ctl->bcount[t] = 0;
-    if (t == 0) {
-        ctl->done_ctas = 0;
-        cc->done_ctas = 0;
-        ctl->n = n;
-        ctl->flat_pct = flat_pct;
-        ctl->ref_intensity = ref_intensity;
-        ctl->mode = kModeWin0;             // the radix passes run only if the windows fail
-        ctl->ntarget = 2;
-    }
-}
-
-// lo/hi from the selected means; bin edges (noise.c:106-119). One block of NT_MAX threads.
-FY_D void k_noise_bins_setup(NoiseCtl* ctl) {
-    fy_pdl_wait();
-    __shared__ double s_lo, s_hi;
-    const int t = threadIdx.x;
-    if (t == 0) {
-        const long long n = ctl->n;
-        const double i1 = 1.0 / 100.0 * (double)(n - 1), i99 = 99.0 / 100.0 * (double)(n - 1);
-        const long long k1 = (long long)i1, k99 = (long long)i99;
-        const double lo = interp(ctl, 0, i1 - (double)k1, k1 + 1 < n);
-        double hi = interp(ctl, 1, i99 - (double)k99, k99 + 1 < n);
-        if (hi <= lo) hi = lo + 1e-6;                   // noise.c:109
-        s_lo = lo;
-        s_hi = hi;
-    }
-    __syncthreads();                                    // targets 0/1 read before they are reset
-    const double lo = s_lo, hi = s_hi;
-    if (t <= NB) {
-        const double e = lo + (hi - lo) * t / NB;      // noise.c:118-119
-        ctl->edge[t] = e;
-        float f = (float)e;
-        if ((double)f < e) f = nextafterf(f, INFINITY);
-        ctl->fedge[t] = f;
-    }
-    // the radix passes' first variance digit: every bin active with the empty prefix (its
-    // histogram gives the bin counts; k_bin_targets then sets the ranks)
-    target_init(ctl, t, 0, 0, t < NB);
-    for (int i = t; i < NB * 3; i += blockDim.x) ctl->bwc[i] = 0;
-    if (t == 0) {
-        ctl->lo = lo;
-        ctl->hi = hi;
-        ctl->fscale = (float)(NB / (hi - lo));
-        ctl->ntarget = NB;
-        // the bins' window runs first (section 2bw); it hands over to the radix passes
-        // (mode 1) when it misses
-        ctl->ncand = 0;
-        ctl->wfail = 0;
-        ctl->mode = kModeBinWin;
-    }
-}
-
-// After the first variance digit pass (one block per bin): the bin's count is the sum of its
-// histogram; targets of the flat_pct percentile for bins with >= 200 voxels (noise.c:123).
-// Bins below that drop out and their histogram is cleared.
-FY_D void k_bin_targets(NoiseCtl* ctl) {
-    fy_pdl_wait();
-    __shared__ unsigned long long part[256];
-    if (ctl->mode != 1) return;
-    const int b = vbx();
-    unsigned int* h = ctl->hist + (size_t)b * 256;
-    part[threadIdx.x] = h[threadIdx.x];
-    __syncthreads();
-    for (int off = 128; off > 0; off >>= 1) {
-        if (threadIdx.x < off) part[threadIdx.x] += part[threadIdx.x + off];
-        __syncthreads();
-    }
-    const long long c = (long long)part[0];
-    const bool on = c >= 200;
-    if (!on) h[threadIdx.x] = 0;
-    if (threadIdx.x == 0) {
-        ctl->bcount[b] = (unsigned long long)c;
-        const double idx = ctl->flat_pct / 100.0 * (double)(c - 1);
-        target_init(ctl, b, on ? (long long)idx : 0, c, on);
-    }
-}
-
-// ---------------------------------------------------------------- 2w. sample-guided window
-// The 1st/99th percentiles of the means by radix selection read the mean field once per
-// digit (3 passes). Here they read it once:
-//   sample   m <= kSampleMax means at positions (A*i + B) mod n, a bijection of [0, n) when
-//            gcd(A, n) = 1, spread evenly over the volume.
-//   window   per target, the sample's order statistics kWinSigmas binomial standard
-//            deviations either side of the target's expected sample rank give a key window
-//            [wlo, whi] that holds the target's order statistics k and k+1 with
-//            overwhelming probability (one CTA per target and window end, radix select in
-//            shared memory to the 24-bit key bucket, widened to its ends).
-//   count    one pass over the means counts, per target, the keys below wlo and appends the
-//            keys inside [wlo, whi] with their target label to a candidate list.
-//   select   the radix passes of mode 1 over the candidates with a second control block,
-//            targets = labels: the first digit pass's per-target sums are the inside counts,
-//            so the target ranks r = k - below are set after it (as the bin counts are in
-//            the bin selection). A rank outside [0, inside) -- k or k+1 not in the window --
-//            or a candidate list over its capacity sends the selection to the radix passes
-//            over the whole field (mode 0), which are exact in every case.
-//   finish   the keys of k and k+1 go into the main block in the form the fit reads.
-// The result is the same exact order statistics as the radix path: only which pass finds
-// them changes. The per-bin variance percentiles use the same scheme (section 2bw).
+// ---------------------------------------------------------------- 2w. sample-guided windows
+// A selection by radix passes alone reads its field once per digit. Here it reads it once:
+//   sample   values at positions (A*i + B) mod n, a bijection of [0, n) when gcd(A, n) = 1,
+//            spread evenly over the volume: 16384 means; 65536 (mean, variance) pairs, listed per
+//            intensity bin.
+//   bounds   per target the sample's order statistics kWinSigmas binomial standard deviations
+//            either side of its expected sample rank give a key window [wlo, whi] that holds the
+//            order statistics k and k+1 with overwhelming probability (block_bounds).
+//   count    one pass over the field(s) counts, per target, the keys below wlo and appends the
+//            keys inside to a candidate list with their target; for the bins it also gives the
+//            bin counts, which set k.
+//   bucket   the candidates' histogram over equal steps of value in the window (a step's bucket
+//            is a monotone function of the key, so buckets are in key order): the bucket of the
+//            rank r = k - below, and of r + 1.
+//   collect  the keys of those buckets (a few hundred; up to kListMax) into a list per target.
+//   select   one CTA per target selects among them in registers.
+// Every step's closing bookkeeping runs in its last CTA. A rank outside its
+// window or a candidate list over its capacity sends the selection to the radix passes over the
+// whole field; buckets with too many keys to collect (ties) send it to the radix passes over the
+// candidates. All of them give the same exact order statistics.
 constexpr int kSampleMax = 16384;
-constexpr int kBoundThreads = 512;
+constexpr int kBinSampleMax = 65536;
+constexpr int kBinListMax = 16384;     // sample keys per bin: a window of 2.4% of the largest bins
+constexpr int kBinListSmall = 2048;    // in the scratch's own region, for fields of few candidates
+constexpr int kListMax = 16384;        // keys that a target can collect
+constexpr int kBoundThreads = 1024;    // CTAs that select among keys in registers
+constexpr int kKeysPerThread = 16;
+static_assert(kSampleMax <= kBoundThreads * kKeysPerThread && kBinListMax <= kBoundThreads * kKeysPerThread &&
+              kListMax <= kBoundThreads * kKeysPerThread, "every list fits the block's registers");
 constexpr double kWinSigmas = 5.0;
 // Test hook: bit 0 forces the mean percentiles, bit 1 the bins, to the radix passes over the
 // whole field; noise_window_used records (bits 0/1) which windows produced their result.
 static __device__ int noise_force_radix;
 static __device__ int noise_window_used;
 
-// Block radix select over keys in shared memory: the rank-th smallest (0-based) of keys[0, c),
-// c <= kSampleMax, by kBoundThreads threads. npass 8-bit digit passes from the top: with
-// npass < 4 the result is the selected key's top 8*npass bits with the rest zero (the bucket
-// that holds it, enough for a window bound). Each warp counts into a
-// private 256-bin histogram (wh, [warps][256]); the lanes of a warp that hold the same digit
-// are merged with __match_any_sync, so one shared atomic counts them all (the high digits of
-// a sample are nearly all equal). Then one thread per digit sums the warps' counts and a
-// warp-shuffle scan over the 256 digit totals finds the bucket of the rank.
-FY_D uint32_t block_select(const uint32_t* keys, int c, long long rank, unsigned int* wh,
-                           unsigned long long* part, uint32_t* s_sel, int npass = 4) {
-    constexpr int NTB = kBoundThreads, NW = NTB / 32;
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+// The bucket that holds rank r in a shared-memory histogram of nh buckets (a power of two, 64 to
+// 2048), and the keys before it; by one warp (every lane gets them; r is below the total). The lanes
+// sum nh/32 buckets each (read rotated: few bank conflicts), then share the rank's segment.
+FY_D void warp_find(const unsigned int* __restrict__ h, int nh, unsigned int r, int& bucket, unsigned int& before) {
     const unsigned full = 0xffffffffu;
-    uint32_t prefix = 0, pmask = 0;
-    unsigned int* mine_h = wh + w * 256;
-    for (int sh = 24; sh >= 32 - 8 * npass; sh -= 8) {
-        for (int i = t; i < NW * 256; i += NTB) wh[i] = 0;
-        __syncthreads();
-        for (int i0 = 0; i0 < c; i0 += NTB) {             // warp-uniform trip count
-            const int i = i0 + t;
-            const uint32_t k = i < c ? keys[i] : 0u;
-            const bool ok = i < c && (k & pmask) == prefix;
-            const unsigned act = __ballot_sync(full, ok);
-            if (ok) {
-                const unsigned d = (k >> sh) & 255u;
-                const unsigned same = __match_any_sync(act, d);
-                if (lane == __ffs(same) - 1) atomicAdd(&mine_h[d], (unsigned)__popc(same));
-            }
-        }
-        __syncthreads();
-        unsigned long long tot = 0;                     // digit t's count over the warps
-        if (t < 256)
-            for (int ww = 0; ww < NW; ++ww) tot += wh[ww * 256 + t];
-        // inclusive scan of the 256 digit totals: within warps by shuffles, then warp sums
-        unsigned long long incl = tot;
+    const int lane = threadIdx.x & 31, per = nh >> 5;
+    auto scan = [&](unsigned int v) {
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(full, incl, o);
-            if (lane >= o) incl += y;
+            const unsigned int y = __shfl_up_sync(full, v, o);
+            if (lane >= o) v += y;
         }
-        if (t < 256 && lane == 31) part[w] = incl;
-        __syncthreads();
-        if (t < 256) {
-            unsigned long long off = 0;
-            for (int ww = 0; ww < w; ++ww) off += part[ww];
-            const unsigned long long hi = off + incl, lo = hi - tot;
-            if ((unsigned long long)rank >= lo && (unsigned long long)rank < hi) {
-                s_sel[0] = (uint32_t)t;
-                s_sel[1] = (uint32_t)(rank - (long long)lo);
-            }
-        }
-        __syncthreads();
-        prefix |= s_sel[0] << sh;
-        pmask |= 255u << sh;
-        rank = s_sel[1];
-        __syncthreads();
-    }
-    return prefix;
+        return v;
+    };
+    unsigned int sum = 0;
+#pragma unroll 8
+    for (int i = 0; i < per; ++i) sum += h[lane * per + ((i + lane) & (per - 1))];
+    unsigned int incl = scan(sum);
+    const int seg = __ffs(__ballot_sync(full, r < incl)) - 1;
+    const unsigned int base = __shfl_sync(full, incl - sum, seg);
+    const unsigned int* hs = h + seg * per;               // at most 64 buckets: two per lane
+    const unsigned int v0 = 2 * lane < per ? hs[2 * lane] : 0u, v1 = 2 * lane + 1 < per ? hs[2 * lane + 1] : 0u;
+    incl = scan(v0 + v1);
+    const int l = __ffs(__ballot_sync(full, r - base < incl)) - 1;
+    unsigned int acc = base + incl - v0 - v1;
+    int b = seg * per + 2 * lane;
+    if (acc + v0 <= r) { acc += v0; ++b; }
+    bucket = __shfl_sync(full, b, l);
+    before = __shfl_sync(full, acc, l);
 }
 
-FY_D void k_win_sample(const float* __restrict__ mean, const NoiseCtl* __restrict__ ctl,
-                                                    float* __restrict__ sm, long long m, unsigned long long A,
-                                                    unsigned long long B) {
-    fy_pdl_wait();
-    if (ctl->mode != kModeWin0) return;
-    const unsigned long long n = (unsigned long long)ctl->n;
-    for (long long i = (long long)vbx() * blockDim.x + threadIdx.x; i < m; i += (long long)vgx() * blockDim.x)
-        sm[i] = __ldg(mean + (A * (unsigned long long)i + B) % n);
-}
-
-// One CTA (kBoundThreads threads) per target (block x 0/1: 1st/99th percentile) and window
-// end (blockIdx.y 0: wlo, 1: whi). Dynamic shared memory: kSampleMax keys, then the warps'
-// digit histograms (kBoundThreads/32 x 256 counters).
-FY_D void k_win_bounds(const float* __restrict__ sm,
-                                                              NoiseCtl* __restrict__ ctl, long long m) {
-    fy_pdl_wait();
-    extern __shared__ uint32_t wkeys[];
-    unsigned int* wh = wkeys + kSampleMax;
-    __shared__ unsigned long long part[kBoundThreads];
-    __shared__ uint32_t s_sel[2];
-    if (ctl->mode != kModeWin0) return;
-    const int t = vbx();
-    const int c = (int)(m < kSampleMax ? m : kSampleMax);
-    for (int i0 = threadIdx.x; i0 < c; i0 += 8 * blockDim.x) {   // eight loads in flight per thread
-        float v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * blockDim.x;
-            v[u] = i < c ? sm[i] : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int i = i0 + u * blockDim.x;
-            if (i < c) wkeys[i] = fkey(v[u]);
-        }
-    }
+// NQ order statistics of the CTA's keys (kKeysPerThread per thread in registers, thread t's i-th is
+// number t + i*kBoundThreads, c >= 1 of them valid; ranks 0-based < c). Histograms of 2048 equal key
+// steps over the keys' range, then inside each rank's bucket: lo <= statistic <= hi, hi - lo below
+// 2^-22 of the range. EXACT: and inside that, lo = statistic. sh: (NQ + 1) * 2048 counters.
+template <int NQ, bool EXACT>
+FY_D void block_stats(const uint32_t (&k)[kKeysPerThread], int c, const int (&rank)[NQ], unsigned int* __restrict__ sh,
+                      uint32_t (&lo)[NQ], uint32_t (&hi)[NQ]) {
+    constexpr int NH = 2048, NTB = kBoundThreads, KPT = kKeysPerThread;
+    __shared__ uint32_t s_min, s_max;
+    __shared__ unsigned int s_b[NQ], s_r[NQ];
+    const unsigned full = 0xffffffffu;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (t == 0) { s_min = 0xffffffffu; s_max = 0u; }
+    for (int i = t; i < (NQ + 1) * NH; i += NTB) sh[i] = 0;
     __syncthreads();
-    const double q = (double)ctl->tk[t] / (double)(ctl->n > 1 ? ctl->n - 1 : 1);   // the target's quantile
-    const bool upper = blockIdx.y == 1;
-    uint32_t w = upper ? 0xffffffffu : 0u;
-    if (c >= 64) {                                      // fewer samples: the whole key range
-        const double qc = q < 1.0 / c ? 1.0 / c : (q > 1.0 - 1.0 / c ? 1.0 - 1.0 / c : q);
-        const long long ks = (long long)(q * (double)(c - 1));
-        const long long d = (long long)ceil(kWinSigmas * sqrt((double)c * qc * (1.0 - qc))) + 4;
-        // three digits: the order statistic's 24-bit key bucket, widened to its ends
-        if (!upper && ks - d >= 0) w = block_select(wkeys, c, ks - d, wh, part, s_sel, 3);
-        if (upper && ks + d + 1 < c) w = block_select(wkeys, c, ks + d + 1, wh, part, s_sel, 3) | 0xffu;
-    }
-    if (threadIdx.x == 0) {
-        if (upper) {
-            ctl->whi[t] = w;
-        } else {
-            ctl->wlo[t] = w;
-            ctl->wbelow[t] = 0;
-            if (t == 0) ctl->ncand = 0;
+    uint32_t mn = 0xffffffffu, mx = 0u;
+#pragma unroll
+    for (int i = 0; i < KPT; ++i)
+        if (t + i * NTB < c) { mn = min(mn, k[i]); mx = max(mx, k[i]); }
+    mn = __reduce_min_sync(full, mn);
+    mx = __reduce_max_sync(full, mx);
+    if (lane == 0 && mn <= mx) { atomicMin(&s_min, mn); atomicMax(&s_max, mx); }
+    __syncthreads();
+    const uint32_t k0 = s_min, range = s_max - k0;
+    const int bits = 32 - __clz(range), sh1 = bits > 11 ? bits - 11 : 0, sh2 = sh1 > 11 ? sh1 - 11 : 0;
+#pragma unroll
+    for (int i = 0; i < KPT; ++i)
+        if (t + i * NTB < c) atomicAdd(&sh[(k[i] - k0) >> sh1], 1u);
+    __syncthreads();
+    auto find = [&](const unsigned int* h, unsigned int r) {    // warp q < NQ
+        int b;
+        unsigned int before;
+        warp_find(h, NH, r, b, before);
+        if (lane == 0) {
+            s_b[w] = (unsigned)b;
+            s_r[w] = r - before;
         }
+    };
+    if (w < NQ) find(sh, (unsigned)rank[w]);
+    __syncthreads();
+    uint32_t pre[NQ];                                    // (key - k0) >> the level's shift, per rank
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) pre[q] = s_b[q];
+    auto level = [&](int from, int to) {                 // refine the buckets of shift `from` to shift `to`
+#pragma unroll
+        for (int i = 0; i < KPT; ++i) {
+            if (t + i * NTB >= c) continue;
+            const uint32_t d = k[i] - k0, b = d >> from, sub = (d & ((1u << from) - 1u)) >> to;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                if (b == pre[q]) atomicAdd(&sh[(q + 1) * NH + sub], 1u);
+        }
+        const unsigned int r = w < NQ ? s_r[w] : 0u;
+        __syncthreads();
+        if (w < NQ) find(sh + (w + 1) * NH, r);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) pre[q] = (pre[q] << (from - to)) + s_b[q];
+    };
+    if (sh1 > 0) level(sh1, sh2);
+    if (EXACT && sh2 > 0) {
+        for (int i = t; i < NQ * NH; i += NTB) sh[NH + i] = 0;
+        __syncthreads();
+        level(sh2, 0);
+    }
+    const int last = EXACT ? 0 : sh2;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        lo[q] = k0 + (pre[q] << last);
+        hi[q] = lo[q] + ((1u << last) - 1u);
     }
 }
 
-// Candidate appends go through a per-warp shared buffer; a full buffer is copied out with one
-// global atomic for its whole run, so the list's counter sees one atomic per ~kWarpBuf
-// candidates instead of one per warp and element.
+// The sample ranks either side of quantile q of c samples (lo < 0 or hi >= c: none).
+FY_D void window_ranks(double q, int c, int& lo, int& hi) {
+    const double qc = q < 1.0 / c ? 1.0 / c : (q > 1.0 - 1.0 / c ? 1.0 - 1.0 / c : q);
+    const int ks = (int)(q * (double)(c - 1));
+    const int d = (int)ceil(kWinSigmas * sqrt((double)c * qc * (1.0 - qc))) + 4;
+    lo = ks - d;
+    hi = ks + d + 1;
+}
+
+// Value buckets of a window: origin and scale of nb equal steps between the sample's keys that
+// bound it (an open window ends at the sample's extremes, so that the bulk of its keys is spread;
+// keys beyond fall into the end buckets). Whatever they are, bucket_of is monotone in the key.
+FY_D void window_buckets(NoiseCtl* ctl, int t, int nb) {
+    const uint32_t kmin = 0x00800000u, kmax = 0xff7fffffu;          // keys of -FLT_MAX and FLT_MAX
+    const uint32_t a = min(max(ctl->klo[t], kmin), kmax), b = min(max(ctl->khi[t], kmin), kmax);
+    const float v0 = funkey(a), d = funkey(b) - v0;
+    ctl->cv0[t] = v0;
+    ctl->cvs[t] = d > 0.f ? (float)nb / d : 0.f;
+}
+FY_D int bucket_of(float v, float v0, float s, int nb) {
+    const int b = (int)((v - v0) * s);                               // saturates; NaN gives 0
+    return fkey(v) > 0xff800000u ? nb - 1 : min(max(b, 0), nb - 1);  // positive NaNs are the largest keys
+}
+
+// One CTA per volume: the control block, and the windows of the 1st/99th percentile of the means.
+FY_D void k_noise_begin(const float* __restrict__ mean, NoiseCtl* __restrict__ ctl, long long n, double flat_pct,
+                        double ref_intensity, unsigned long long A, unsigned long long B, unsigned long long step) {
+    fy_pdl_wait();
+    extern __shared__ unsigned int wsh[];                // 5 * 2048 counters
+    const int t = threadIdx.x;
+    const int c = (int)(n < kSampleMax ? n : kSampleMax);
+    uint32_t k[kKeysPerThread];
+    unsigned long long pos = (A * (unsigned long long)t + B) % (unsigned long long)n;   // step = A*kBoundThreads mod n
+#pragma unroll
+    for (int i = 0; i < kKeysPerThread; ++i) {
+        k[i] = t + i * kBoundThreads < c ? fkey(__ldg(mean + pos)) : 0u;
+        pos += step;
+        if (pos >= (unsigned long long)n) pos -= (unsigned long long)n;
+    }
+    static_assert(sizeof(ctl->hist) % 16 == 0 && offsetof(NoiseCtl, hist) % 16 == 0, "uint4 clears");
+    for (int i = t; i < (int)(sizeof(ctl->hist) / 16); i += kBoundThreads)
+        reinterpret_cast<uint4*>(ctl->hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    const double i1 = 1.0 / 100.0 * (double)(n - 1), i99 = 99.0 / 100.0 * (double)(n - 1);
+    const long long k1 = (long long)i1, k99 = (long long)i99;
+    if (t < NB) {
+        target_init(ctl, t, t == 0 ? k1 : (t == 1 ? k99 : 0), n, t < 2);
+        ctl->wbelow[t] = ctl->wvox[t] = ctl->bcount[t] = 0;
+        ctl->ccnt[t] = ctl->bsn[t] = 0;
+        ctl->wlo[t] = ctl->klo[t] = 0u;
+        ctl->whi[t] = ctl->khi[t] = 0xffffffffu;
+    }
+    if (t == 0) {
+        ctl->n = n;
+        ctl->flat_pct = flat_pct;
+        ctl->ref_intensity = ref_intensity;
+        ctl->ntarget = 2;
+        ctl->done_ctas = 0;
+        ctl->ncand = 0;
+        ctl->mode = kMeanWin;
+    }
+    if (c < 64) return;                                  // every key is a candidate
+    const double nm = (double)(n > 1 ? n - 1 : 1);
+    int lo0, hi0, lo1, hi1;
+    window_ranks((double)k1 / nm, c, lo0, hi0);
+    window_ranks((double)k99 / nm, c, lo1, hi1);
+    const int rank[4] = {max(lo0, 0), min(hi0, c - 1), max(lo1, 0), min(hi1, c - 1)};
+    uint32_t lo[4], hi[4];
+    block_stats<4, false>(k, c, rank, wsh, lo, hi);
+    if (t == 0) {
+        ctl->klo[0] = lo[0]; ctl->khi[0] = hi[1];
+        ctl->klo[1] = lo[2]; ctl->khi[1] = hi[3];
+        if (lo0 >= 0) ctl->wlo[0] = lo[0];
+        if (hi0 < c) ctl->whi[0] = hi[1];
+        if (lo1 >= 0) ctl->wlo[1] = lo[2];
+        if (hi1 < c) ctl->whi[1] = hi[3];
+    }
+}
+
+// Buckets per target. The bins' windows hold nearly equal numbers of candidates (a bin's sample grows
+// with it): at 512^3 60,000 to 700,000 each, so 300 to 6,000 keys a bucket.
+constexpr int kMeanBuckets = 2048, kBinBuckets = 256;
+static_assert(2 * kMeanBuckets <= kHist && NB * kBinBuckets <= kHist, "the control block's histogram holds them");
 
 // The counting pass: mean keys against the windows of targets 0 and 1. The counts below each
 // window stay in registers until one warp reduction at the end; the keys inside a window go
@@ -831,7 +621,6 @@ FY_D void k_win_count(const float* __restrict__ mean, NoiseCtl* __restrict__ ctl
     static_assert(32 * 4 * SU * 2 <= kCountBuf, "one step must fit the warp buffer");
     __shared__ float bufv[256 / 32][kCountBuf];
     __shared__ uint8_t bufl[256 / 32][kCountBuf];
-    if (ctl->mode != kModeWin0) return;
     const unsigned full = 0xffffffffu;
     const int t = threadIdx.x, lane = t & 31;
     WarpCands wc;
@@ -915,269 +704,281 @@ FY_D void k_win_count(const float* __restrict__ mean, NoiseCtl* __restrict__ ctl
         if (s0) atomicAdd(&ctl->wbelow[0], (unsigned long long)s0);
         if (s1) atomicAdd(&ctl->wbelow[1], (unsigned long long)s1);
     }
-}
-
-// After the counting pass (one thread): arms the candidate block for its first digit pass
-// (both targets active with the empty prefix, like the bin selection's labelling pass), or,
-// when the candidate list overflowed, sends the selection to the radix passes.
-FY_D void k_win_arm(NoiseCtl* __restrict__ ctl, NoiseCtl* __restrict__ cc, long long cap) {
-    fy_pdl_wait();
-    if (ctl->mode != kModeWin0) { cc->mode = 3; return; }
-    for (int t = 0; t < NT_MAX; ++t) target_init(cc, t, 0, 0, t < 2);
-    cc->ntarget = 2;
-    cc->n = (long long)(ctl->ncand < (unsigned long long)cap ? ctl->ncand : (unsigned long long)cap);
-    ctl->wfail = 0;
-    if ((long long)ctl->ncand > cap || (noise_force_radix & 1)) {
-        cc->mode = 3;
-        ctl->wfail = 1;
-        ctl->mode = 0;                     // the radix passes over the whole field
-    } else {
-        cc->mode = 1;
+    if (!last_cta(ctl)) return;
+    if (t < 2) window_buckets(ctl, t, kMeanBuckets);
+    if (t == 0) {
+        ctl->done_ctas = 0;
+        if ((long long)__ldcg(&ctl->ncand) > cap || (noise_force_radix & 1)) ctl->mode = kMeanField;
     }
 }
 
-// After the candidates' first digit pass (one block per target): the target's inside count
-// is the sum of its histogram; its rank among the candidates is r = k - below, which must
-// leave k and (when it exists) k+1 inside. Otherwise the window failed: the candidate passes
-// stand aside (cc mode 3) and the radix passes over the whole field run (mode 0). A block
-// that finds cc already failed leaves its histogram, which every later user clears first.
-FY_D void k_win_targets(NoiseCtl* __restrict__ ctl, NoiseCtl* __restrict__ cc) {
-    fy_pdl_wait();
-    __shared__ unsigned long long part[256];
-    if (cc->mode != 1) return;
-    const int t = vbx();
-    if (t >= cc->ntarget) return;
-    unsigned int* h = cc->hist + (size_t)t * 256;
-    part[threadIdx.x] = h[threadIdx.x];
-    __syncthreads();
-    for (int off = 128; off > 0; off >>= 1) {
-        if (threadIdx.x < off) part[threadIdx.x] += part[threadIdx.x + off];
-        __syncthreads();
+// f(value, target) for a thread's share of the candidates, U quads in flight at a time (collecting
+// the bins' 39 MB of candidates at 512^3 takes 30 us with U = 1, 24 with 4; bucketing, whose shared
+// atomics bound it, 24 with 1, 28 with 4).
+template <int U, class F>
+FY_D void for_each_cand(const NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab, F f) {
+    const long long n = (long long)ctl->ncand, n4f = n / 4;
+    const long long stride = (long long)vgx() * blockDim.x, i0 = (long long)vbx() * blockDim.x + threadIdx.x;
+    for (long long q = i0; q < n4f; q += U * stride) {
+        float4 x[U];
+        uchar4 g[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (q + u * stride < n4f) {
+                x[u] = *(reinterpret_cast<const float4*>(cval) + q + u * stride);
+                g[u] = *(reinterpret_cast<const uchar4*>(clab) + q + u * stride);
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (q + u * stride < n4f) {
+                f(x[u].x, g[u].x);
+                f(x[u].y, g[u].y);
+                f(x[u].z, g[u].z);
+                f(x[u].w, g[u].w);
+            }
     }
-    const long long in = (long long)part[0];
-    const long long k = ctl->tk[t];
-    const long long r = k - (long long)ctl->wbelow[t];
-    const bool has_next = k + 1 < ctl->n;
-    const bool ok = r >= 0 && r < in && (!has_next || r + 1 < in);
+    for (long long i = 4 * n4f + i0; i < n; i += stride) f(cval[i], clab[i]);
+}
+
+// Bucket step for nt targets of nb buckets: the candidates' histogram; the last CTA finds per target the buckets
+// of r = k - below and r + 1. `field` and `cand`: the modes of the radix passes that take over;
+// lcap: keys that a target can collect.
+FY_D void cand_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab, int nt,
+                      int nb, long long lcap, int field, int cand) {
+    extern __shared__ unsigned int rh[];
+    __shared__ float sv0[NB], svs[NB];
+    __shared__ int s_field, s_cand;
+    const int t = threadIdx.x, lane = t & 31;
+    const unsigned full = 0xffffffffu;
+    for (int i = t; i < nt * nb; i += blockDim.x) rh[i] = 0;
+    if (t < nt) { sv0[t] = ctl->cv0[t]; svs[t] = ctl->cvs[t]; }
+    if (t == 0) s_field = s_cand = 0;
     __syncthreads();
-    if (!ok) h[threadIdx.x] = 0;                         // inactive: its histogram is cleared
-    if (threadIdx.x == 0) {
-        target_init(cc, t, ok ? r : 0, in, ok);
-        if (!ok) {
-            ctl->wfail = 1;
-            cc->mode = 3;
-            ctl->mode = 0;
+    auto count = [&](float v, int g) { atomicAdd(&rh[g * nb + bucket_of(v, sv0[g], svs[g], nb)], 1u); };
+    for_each_cand<1>(ctl, cval, clab, count);
+    __syncthreads();
+#pragma unroll 4
+    for (int i = t; i < nt * nb; i += blockDim.x)
+        if (rh[i]) atomicAdd(&ctl->hist[i], rh[i]);
+    if (!last_cta(ctl)) return;
+#pragma unroll 4
+    for (int i = t; i < nt * nb; i += blockDim.x) {
+        rh[i] = __ldcg(&ctl->hist[i]);
+        ctl->hist[i] = 0;
+    }
+    __syncthreads();
+    for (int g = t >> 5; g < nt; g += blockDim.x >> 5) {
+        if (!ctl->tactive[g]) continue;
+        const unsigned int* h = rh + g * nb;
+        unsigned int total = 0;
+        for (int i = lane; i < nb; i += 32) total += h[i];
+        total = __reduce_add_sync(full, total);
+        const long long k = ctl->tk[g], r = k - (long long)__ldcg(&ctl->wbelow[g]);
+        const bool has_next = k + 1 < ctl->tgroup_n[g];
+        if (!(r >= 0 && r < (long long)total && (!has_next || r + 1 < (long long)total))) {
+            if (lane == 0) s_field = 1;
+            continue;
+        }
+        int b0, b1;
+        unsigned int before, before1;
+        warp_find(h, nb, (unsigned)r, b0, before);
+        b1 = b0;
+        if (has_next) warp_find(h, nb, (unsigned)r + 1u, b1, before1);
+        if (lane == 0) {
+            const long long cnt = (long long)h[b0] + (b1 != b0 ? h[b1] : 0u);
+            ctl->cb0[g] = b0;
+            ctl->cb1[g] = b1;
+            ctl->crank[g] = r - (long long)before;
+            ctl->trank[g] = r;                            // for the radix passes over the candidates
+            if (cnt > lcap) s_cand = 1;
         }
     }
-}
-
-// The bins' candidate list (section 2b). Reset before the compacting pass.
-FY_D void k_bin_cand_reset(NoiseCtl* __restrict__ ctl) {
-    fy_pdl_wait();
-    if (ctl->mode == 1) ctl->ncand = 0;
-}
-// After the compacting pass and its scan: when the list fits, the bins' targets move to the
-// candidate block for the last digit and the whole-field pass stands aside; otherwise the
-// candidate pass stands aside.
-FY_D void k_bin_arm(NoiseCtl* __restrict__ ctl, NoiseCtl* __restrict__ cc, long long cap) {
-    fy_pdl_wait();
-    __shared__ int s_go;
-    if (threadIdx.x == 0) s_go = ctl->mode == 1 && (long long)ctl->ncand <= cap;
     __syncthreads();
-    if (!s_go) {
-        if (threadIdx.x == 0) cc->mode = 3;
-        return;
+    if (t < nt && s_field) ctl->trank[t] = ctl->tk[t];
+    if (t == 0) {
+        ctl->done_ctas = 0;
+        if (s_field) ctl->mode = field;
+        else if (s_cand) ctl->mode = cand;
     }
-    for (int i = threadIdx.x; i < NB * 256; i += blockDim.x) cc->hist[i] = 0;
-    for (int t = threadIdx.x; t < NT_MAX; t += blockDim.x) {
-        cc->tk[t] = ctl->tk[t];
-        cc->trank[t] = ctl->trank[t];
-        cc->tgroup_n[t] = ctl->tgroup_n[t];
-        cc->tprefix[t] = ctl->tprefix[t];
-        cc->tactive[t] = ctl->tactive[t];
-        cc->teq[t] = 0;
-        cc->tneed_next[t] = 0;
-        cc->tnext[t] = 0xffffffffu;
+}
+
+// Collect step: the candidates in their target's buckets into its list (the bucket step bounded
+// their number by lcap). A CTA's hits wait in shared memory, so that each target's counter takes one
+// atomic per CTA (one per key, 60,000 keys on 24 counters at 512^3, took 8 us more).
+constexpr int kCollectBuf = 1024;
+FY_D void cand_collect(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab, int nt,
+                       int nb, uint32_t* __restrict__ list, long long lcap) {
+    __shared__ float sv0[NB], svs[NB];
+    __shared__ int sb0[NB], sb1[NB];
+    __shared__ unsigned int scnt[NB], sbase[NB], s_fill;
+    __shared__ uint2 buf[kCollectBuf];                   // key; target << 16 | its place among the CTA's
+    const int t = threadIdx.x;
+    if (t < nt) {
+        sv0[t] = ctl->cv0[t];
+        svs[t] = ctl->cvs[t];
+        sb0[t] = ctl->tactive[t] ? ctl->cb0[t] : -1;
+        sb1[t] = ctl->tactive[t] ? ctl->cb1[t] : -1;
+        scnt[t] = 0;
     }
+    if (t == 0) s_fill = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        cc->n = (long long)ctl->ncand;
-        cc->ntarget = ctl->ntarget;
-        cc->mode = 1;
-        ctl->mode = kModeBinCand;
-    }
-}
-// After the candidates' last digit: the selected keys back into the main block.
-FY_D void k_bin_finish(NoiseCtl* __restrict__ ctl, const NoiseCtl* __restrict__ cc) {
-    fy_pdl_wait();
-    if (ctl->mode != kModeBinCand) return;
-    for (int t = 0; t < NT_MAX; ++t) {
-        ctl->tprefix[t] = cc->tprefix[t];
-        ctl->trank[t] = cc->trank[t];
-        ctl->teq[t] = cc->teq[t];
-        ctl->tneed_next[t] = cc->tneed_next[t];
-        ctl->tnext[t] = cc->tnext[t];
-    }
-    ctl->mode = 1;
-}
-
-// Keys of order statistics k and k+1 into the main block's targets 0/1 (interp / next_value
-// form); the radix passes of mode 0 then stand aside.
-FY_D void k_win_finish(NoiseCtl* __restrict__ ctl, const NoiseCtl* __restrict__ cc) {
-    fy_pdl_wait();
-    if (ctl->mode != kModeWin0) return;
-    for (int t = 0; t < 2; ++t) {
-        ctl->tprefix[t] = cc->tprefix[t];
-        ctl->tnext[t] = cc->tneed_next[t] ? cc->tnext[t] : cc->tprefix[t];
-        ctl->tneed_next[t] = 1;
-        ctl->tactive[t] = 1;
-    }
-    atomicOr(&noise_window_used, 1);
-}
-
-// ---------------------------------------------------------------- 2bw. the bins' window
-// The flat_pct percentile of the variance per intensity bin by the scheme of section 2w,
-// so the variance field is read once instead of once per digit:
-//   sample   m (<= kBinSampleMax) voxels at positions (A*i + B) mod n: the key of each
-//            variance and the bin of its mean (255: outside every bin).
-//   window   one CTA per bin gathers the bin's sample keys in sample order (at most
-//            kBinKeysMax) and takes the order statistics kWinSigmas binomial standard
-//            deviations either side of the target's sample rank, each widened to its 16-bit
-//            key bucket (two digit passes): [bwlo, bwhi]. Under 64 samples: every key.
-//   count    one branch-free pass over mean and variance: per bin its voxels (the bin count,
-//            noise.c:118-123) and the keys below its window; the keys inside go to the
-//            candidate list with their bin.
-//   arm      for each bin of >= 200 voxels, r = k - below with k = flat_pct/100*(count - 1);
-//            the first digit pass over the candidates (control block cc, targets = bins) gives
-//            the inside counts, and k and k+1 must be inside (k_bwin_targets); the other three
-//            digit passes then select them. A miss, an overfull list or a failed bin guess
-//            sends the bins to the radix passes over the whole field (mode 1).
-//   finish   the keys of k and k+1 into the main block; mode kModeBinDone makes the radix
-//            passes stand aside.
-constexpr int kBinSampleMax = 65536;
-constexpr int kBinKeysMax = 4096;      // per bin: enough for a window of ~5% of a large bin
-
-FY_D void k_bwin_sample(const float* __restrict__ mean, const float* __restrict__ var,
-                                                     const NoiseCtl* __restrict__ ctl, uint32_t* __restrict__ skey,
-                                                     uint8_t* __restrict__ slab, long long m, unsigned long long A,
-                                                     unsigned long long B) {
-    fy_pdl_wait();
-    __shared__ float fe[NB + 1];
-    if (ctl->mode != kModeBinWin) return;
-    if (threadIdx.x <= NB) fe[threadIdx.x] = ctl->fedge[threadIdx.x];
-    __syncthreads();
-    const float lo_f = fe[0], fscale = ctl->fscale;
-    const unsigned long long n = (unsigned long long)ctl->n;
-    for (long long i = (long long)vbx() * blockDim.x + threadIdx.x; i < m; i += (long long)vgx() * blockDim.x) {
-        const unsigned long long q = (A * (unsigned long long)i + B) % n;
-        const float mv = __ldg(mean + q), vv = __ldg(var + q);
-        const int b = bin_of(mv, fe, lo_f, fscale);
-        skey[i] = fkey(vv);
-        slab[i] = (uint8_t)(b < 0 ? 255 : b);
-    }
-}
-
-// One CTA (kBoundThreads threads) per bin. Dynamic shared memory as k_win_bounds. Each warp
-// owns a contiguous slice of the sample (whole 512-entry steps, 16 labels per lane and step,
-// read 16 bytes at a time, the next step's while the current one is placed) and compacts its
-// bin's keys in sample order into its own kBinKeysMax/NW slots, with no block barrier; one
-// block pass then concatenates the warps' keys (a deterministic subset in sample order).
-FY_D void k_bwin_bounds(const uint32_t* __restrict__ skey,
-                                                               const uint8_t* __restrict__ slab,
-                                                               NoiseCtl* __restrict__ ctl, long long m) {
-    fy_pdl_wait();
-    constexpr int NTB = kBoundThreads, NW = NTB / 32, U = 16, STEP = 32 * U, WCAP = kBinKeysMax / NW;
-    static_assert(2 * kBinKeysMax <= kSampleMax, "staging and compacted keys share the key array");
-    extern __shared__ uint32_t wkeys[];
-    unsigned int* wh = wkeys + kSampleMax;
-    uint32_t* keys = wkeys + kBinKeysMax;                 // the concatenated keys
-    __shared__ unsigned long long part[NTB];
-    __shared__ uint32_t s_sel[2];
-    __shared__ int s_wc[NW];
-    if (ctl->mode != kModeBinWin) return;
-    const int b = vbx(), t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const unsigned full = 0xffffffffu;
-    auto load_labels = [&](long long e0, uint8_t* lab) {
-        if (e0 + U <= m) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(slab + e0));
-            const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < U; ++j) lab[j] = (uint8_t)(wv[j >> 2] >> (8 * (j & 3)));
-        } else {
-#pragma unroll
-            for (int j = 0; j < U; ++j) lab[j] = e0 + j < m ? slab[e0 + j] : (uint8_t)255;
+    auto visit = [&](float v, int g) {
+        const int b = bucket_of(v, sv0[g], svs[g], nb);
+        if (b != sb0[g] && b != sb1[g]) return;
+        const unsigned int f = atomicAdd(&s_fill, 1u);
+        if (f < (unsigned)kCollectBuf) {
+            buf[f] = make_uint2(fkey(v), (unsigned)g << 16 | atomicAdd(&scnt[g], 1u));
+        } else {                                         // the buffer is full: straight to the list
+            const unsigned int pos = atomicAdd(&ctl->ccnt[g], 1u);
+            if (pos < lcap) list[g * lcap + pos] = fkey(v);
         }
     };
-    // this warp's slice: whole steps, so every 16-label read is 16-byte aligned
-    const long long steps = (m + STEP - 1) / STEP, per = (steps + NW - 1) / NW;
-    const long long s0 = (long long)w * per * STEP, s1 = s0 + per * STEP < m ? s0 + per * STEP : m;
-    uint32_t* mine = wkeys + w * WCAP;
-    int wc = 0;                                           // warp-uniform
-    uint8_t nxt[U];
-    if (s0 < s1) load_labels(s0 + lane * U, nxt);
-    for (long long i0 = s0; i0 < s1 && wc < WCAP; i0 += STEP) {
-        uint8_t lab[U];
+    for_each_cand<4>(ctl, cval, clab, visit);
+    __syncthreads();
+    if (t < nt && scnt[t]) sbase[t] = atomicAdd(&ctl->ccnt[t], scnt[t]);
+    __syncthreads();
+    const int fill = (int)min(s_fill, (unsigned)kCollectBuf);
+    for (int i = t; i < fill; i += blockDim.x) {
+        const unsigned int g = buf[i].y >> 16, pos = sbase[g] + (buf[i].y & 0xffffu);
+        if (pos < lcap) list[g * lcap + pos] = buf[i].x;
+    }
+}
+// Select step: one CTA per target selects the keys of k and k+1 among those collected.
+FY_D void k_cand_select(NoiseCtl* __restrict__ ctl, const uint32_t* __restrict__ list, long long lcap, int win, int cand,
+                        int used_bit) {
+    fy_pdl_wait();
+    extern __shared__ unsigned int wsh[];                // 3 * 2048 counters
+    const int g = vbx(), t = threadIdx.x, mode = ctl->mode;
+    if (t == 0 && g == 0 && (mode == win || mode == cand)) atomicOr(&noise_window_used, used_bit);
+    if (mode != win || g >= ctl->ntarget || !ctl->tactive[g]) return;
+    const int c = (int)ctl->ccnt[g], r = (int)ctl->crank[g];
+    const bool has_next = ctl->tk[g] + 1 < ctl->tgroup_n[g];
+    uint32_t k[kKeysPerThread];
 #pragma unroll
-        for (int j = 0; j < U; ++j) lab[j] = nxt[j];
-        const long long e0 = i0 + lane * U;
-        if (i0 + STEP < s1) load_labels(e0 + STEP, nxt);
-        unsigned hit = 0;
-#pragma unroll
-        for (int j = 0; j < U; ++j) hit |= (unsigned)(lab[j] == (uint8_t)b && e0 + j < s1) << j;
-        const int cnt = __popc(hit);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(full, incl, o);
-            if (lane >= o) incl += y;
+    for (int i = 0; i < kKeysPerThread; ++i)
+        k[i] = t + i * kBoundThreads < c ? list[g * lcap + t + i * kBoundThreads] : 0u;
+    const int rank[2] = {r, has_next ? r + 1 : r};
+    uint32_t lo[2], hi[2];
+    block_stats<2, true>(k, c, rank, wsh, lo, hi);
+    if (t == 0) {
+        ctl->tprefix[g] = lo[0];
+        ctl->tnext[g] = lo[1];
+        ctl->tneed_next[g] = has_next;
+        ctl->ccnt[g] = 0;
+    }
+}
+
+FY_D void k_mean_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
+                        long long lcap) {
+    fy_pdl_wait();
+    if (ctl->mode == kMeanWin) cand_bucket(ctl, cval, clab, 2, kMeanBuckets, lcap, kMeanField, kMeanCand);
+}
+FY_D void k_mean_collect(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
+                         uint32_t* __restrict__ list, long long lcap) {
+    fy_pdl_wait();
+    if (ctl->mode == kMeanWin) cand_collect(ctl, cval, clab, 2, kMeanBuckets, list, lcap);
+}
+FY_D void k_bin_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
+                       long long lcap) {
+    fy_pdl_wait();
+    if (ctl->mode == kBinWin) cand_bucket(ctl, cval, clab, NB, kBinBuckets, lcap, kBinField, kBinCand);
+}
+FY_D void k_bin_collect(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
+                        uint32_t* __restrict__ list, long long lcap) {
+    fy_pdl_wait();
+    if (ctl->mode == kBinWin) cand_collect(ctl, cval, clab, NB, kBinBuckets, list, lcap);
+}
+
+// The bins: lo/hi from the selected means and the bin edges (noise.c:106-119), which every CTA
+// forms for itself and one writes down; then the sample, each (mean, variance) pair's variance key
+// listed under the bin of its mean (a CTA's keys of a bin take one atomic).
+constexpr int kBinSampleThreads = 512;
+FY_D void k_bin_sample(const float* __restrict__ mean, const float* __restrict__ var, NoiseCtl* __restrict__ ctl,
+                       uint32_t* __restrict__ list, int lcap, long long m, unsigned long long A, unsigned long long B) {
+    fy_pdl_wait();
+    __shared__ float fe[NB + 1];
+    __shared__ double s_lo, s_hi;
+    __shared__ unsigned int scnt[NB], sbase[NB];
+    const int t = threadIdx.x;
+    const unsigned long long n = (unsigned long long)ctl->n;
+    if (t == 0) {
+        const double i1 = 1.0 / 100.0 * (double)(n - 1), i99 = 99.0 / 100.0 * (double)(n - 1);
+        const long long k1 = (long long)i1, k99 = (long long)i99;
+        const double lo = interp(ctl, 0, i1 - (double)k1, k1 + 1 < (long long)n);
+        double hi = interp(ctl, 1, i99 - (double)k99, k99 + 1 < (long long)n);
+        if (hi <= lo) hi = lo + 1e-6;                    // noise.c:109
+        s_lo = lo;
+        s_hi = hi;
+    }
+    if (t < NB) scnt[t] = 0;
+    __syncthreads();
+    if (t <= NB) {
+        const double e = s_lo + (s_hi - s_lo) * t / NB;  // noise.c:118-119
+        float f = (float)e;
+        if ((double)f < e) f = nextafterf(f, INFINITY);
+        fe[t] = f;
+        if (vbx() == 0) {
+            ctl->edge[t] = e;
+            ctl->fedge[t] = f;
         }
-        int pos = wc + incl - cnt;
-#pragma unroll
-        for (int j = 0; j < U; ++j)
-            if ((hit >> j) & 1u) {
-                if (pos < WCAP) mine[pos] = __ldg(skey + e0 + j);
-                ++pos;
-            }
-        const int tot = __shfl_sync(full, incl, 31);
-        wc = wc + tot < WCAP ? wc + tot : WCAP;
     }
-    if (lane == 0) s_wc[w] = wc;
-    __syncthreads();
-    int off = 0, c = 0;
-#pragma unroll
-    for (int ww = 0; ww < NW; ++ww) {
-        const int v = s_wc[ww];
-        off += ww < w ? v : 0;
-        c += v;
+    if (vbx() == 0) {                                    // no CTA of this step reads these
+        if (t < NB) ctl->wbelow[t] = ctl->wvox[t] = 0;
+        if (t == 0) ctl->ncand = 0;
     }
-    for (int i = lane; i < wc; i += 32) keys[off + i] = mine[i];
     __syncthreads();
-    uint32_t lo = 0u, hi = 0xffffffffu;
-    if (c >= 64) {
-        const double q = ctl->flat_pct / 100.0;
-        const double qc = q < 1.0 / c ? 1.0 / c : (q > 1.0 - 1.0 / c ? 1.0 - 1.0 / c : q);
-        const long long ks = (long long)(q * (double)(c - 1));
-        const long long d = (long long)ceil(kWinSigmas * sqrt((double)c * qc * (1.0 - qc))) + 4;
-        if (ks - d >= 0) lo = block_select(keys, c, ks - d, wh, part, s_sel, 2);
-        if (ks + d + 1 < c) hi = block_select(keys, c, ks + d + 1, wh, part, s_sel, 2) | 0xffffu;
+    const float lo_f = fe[0], fscale = (float)(NB / (s_hi - s_lo));
+    const long long i = (long long)vbx() * blockDim.x + t;    // one sample per thread
+    int b = -1;
+    uint32_t key = 0;
+    unsigned int pos = 0;
+    if (i < m) {
+        const unsigned long long q = (A * (unsigned long long)i + B) % n;
+        const float mv = __ldg(mean + q), vv = __ldg(var + q);
+        b = bin_of(mv, fe, lo_f, fscale);
+        key = fkey(vv);
+        if (b >= 0) pos = atomicAdd(&scnt[b], 1u);
+    }
+    __syncthreads();
+    if (t < NB && scnt[t]) sbase[t] = atomicAdd(&ctl->bsn[t], scnt[t]);
+    __syncthreads();
+    if (b >= 0 && sbase[b] + pos < (unsigned)lcap) list[(size_t)b * lcap + sbase[b] + pos] = key;
+}
+
+// One CTA per bin: the window of its flat_pct percentile from its listed sample.
+FY_D void k_bin_bounds(const uint32_t* __restrict__ list, int lcap, NoiseCtl* __restrict__ ctl) {
+    fy_pdl_wait();
+    extern __shared__ unsigned int wsh[];                // 3 * 2048 counters
+    const int b = vbx(), t = threadIdx.x;
+    const int c = (int)min(ctl->bsn[b], (unsigned)lcap);
+    uint32_t k[kKeysPerThread];
+#pragma unroll
+    for (int i = 0; i < kKeysPerThread; ++i) k[i] = t + i * kBoundThreads < c ? list[(size_t)b * lcap + t + i * kBoundThreads] : 0u;
+    uint32_t kl[2] = {0u, 0u}, kh[2] = {0xffffffffu, 0xffffffffu};
+    int lo = -1, hi = c;
+    if (c > 0) {
+        if (c >= 64) window_ranks(ctl->flat_pct / 100.0, c, lo, hi);
+        const int rank[2] = {min(max(lo, 0), c - 1), min(max(hi, 0), c - 1)};
+        block_stats<2, false>(k, c, rank, wsh, kl, kh);
     }
     if (t == 0) {
-        ctl->bwlo[b] = lo;
-        ctl->bwhi[b] = hi;
+        ctl->klo[b] = kl[0];
+        ctl->khi[b] = kh[1];
+        ctl->wlo[b] = lo >= 0 && lo < c ? kl[0] : 0u;             // no sample below (above): open
+        ctl->whi[b] = hi >= 0 && hi < c ? kh[1] : 0xffffffffu;
     }
 }
 
 // The counting pass of the bins' windows: mean and variance read once, SUB float4 of each
 // per thread and step. Every voxel takes the same branch-free path: its bin from the float
-// guess corrected by one step (exact unless the range [lo, hi] is degenerate; a voxel whose
-// corrected bin fails the exact membership test raises ctl->wfail and the bins fall back to
-// the radix passes), the key of its variance against the bin's window, and one
-// read-modify-write of the lane's own shared-memory counter of its bin (low 16 bits: the
-// bin's voxels, high 16 bits: those below the window; rows of 25 words, so the lanes of a
-// warp hit distinct banks when they share a bin; added into the CTA's totals before a field
-// can pass 65535). The keys inside the window are placed by one warp scan per step in the
-// warp's buffer and appended to the list (one atomic per buffer), as in k_win_count. The
-// inside counts come from the candidates' first digit histogram (k_bwin_targets).
+// guess (one 16-byte lookup gives the guessed bin's edges and window; when the mean lies outside
+// the guess, by rounding at an edge or in a degenerate range, the exact walk corrects it), the
+// key of its variance against the bin's window, and one read-modify-write of the lane's own
+// shared-memory counter of its bin (low 16 bits: the bin's voxels, high 16 bits: those below the
+// window; rows of 25 words, so the lanes of a warp hit distinct banks when they share a bin;
+// added into the CTA's totals before a field can pass 65535). The keys inside the window are
+// placed by one warp scan per step in the warp's buffer and appended to the list (one atomic per
+// buffer), as in k_win_count. The last CTA sets the bins' ranks from the counts.
 constexpr int kBCountBuf = 512;          // per warp: two steps' worst case (32 x 8 each)
 constexpr int kLaneRow = 25;             // counter words per lane (NB = 24, odd stride)
 FY_D void k_bwin_count(const float* __restrict__ mean, const float* __restrict__ var,
@@ -1190,62 +991,49 @@ FY_D void k_bwin_count(const float* __restrict__ mean, const float* __restrict__
     __shared__ uint8_t bufl[256 / 32][kBCountBuf];
     __shared__ unsigned int lc[256 * kLaneRow];          // per-lane counters
     __shared__ float fe[NB + 1];
-    __shared__ uint32_t swl[NB], swh[NB];
     __shared__ float4 stab[NB];                          // per bin: its edges and its window
-    __shared__ unsigned int sc[NB * 3];
-    __shared__ int s_bad;
-    if (ctl->mode != kModeBinWin) return;
+    __shared__ unsigned int sc[NB * 2];
     const unsigned full = 0xffffffffu;
     const int t = threadIdx.x, lane = t & 31;
     if (t <= NB) fe[t] = ctl->fedge[t];
-    if (t < NB) {
-        const uint32_t wl = ctl->bwlo[t], wh = ctl->bwhi[t];
-        swl[t] = wl;
-        swh[t] = wh;
-        stab[t] = make_float4(ctl->fedge[t], ctl->fedge[t + 1], __uint_as_float(wl), __uint_as_float(wh));
-    }
-    for (int i = t; i < NB * 3; i += blockDim.x) sc[i] = 0;
+    if (t < NB)
+        stab[t] = make_float4(ctl->fedge[t], ctl->fedge[t + 1], __uint_as_float(ctl->wlo[t]), __uint_as_float(ctl->whi[t]));
+    for (int i = t; i < NB * 2; i += blockDim.x) sc[i] = 0;
     for (int i = t; i < 256 * kLaneRow; i += blockDim.x) lc[i] = 0;
-    if (t == 0) s_bad = 0;
     __syncthreads();
-    const float lo_e = fe[0], hi_e = fe[NB], fscale = ctl->fscale;
+    const float lo_e = fe[0], hi_e = fe[NB], fscale = (float)(NB / (ctl->edge[NB] - ctl->edge[0]));
     unsigned int* row = lc + t * kLaneRow;
     WarpCands wc;
     wc.v = bufv[t >> 5];
     wc.l = bufl[t >> 5];
-    bool bad = false;
-    // bin (or -1 outside every bin) and whether the key is inside the bin's window. One
-    // 16-byte lookup gives the guessed bin's edges and window; when the mean lies outside the
-    // guess (rare: rounding at an edge), one step to the neighbour and the exact-membership
-    // check of the step run as before.
+    // bin (or -1 outside every bin) and whether the key is inside the bin's window
     auto classify = [&](float m, float v, bool valid, int& bo, bool& inside) {
         const bool inr = valid && m >= lo_e && m < hi_e;
         const float mc = inr ? m : lo_e;
         int b = (int)((mc - lo_e) * fscale);
         b = b < 0 ? 0 : (b > NB - 1 ? NB - 1 : b);
-        const float4 e = stab[b];
-        uint32_t wl = __float_as_uint(e.z), wh = __float_as_uint(e.w);
+        float4 e = stab[b];
         if (!(mc >= e.x && mc < e.y)) {
-            b = b - (int)(mc < e.x) + (int)(mc >= e.y);
-            bad |= !(mc >= fe[b] && mc < fe[b + 1]);
-            wl = swl[b];
-            wh = swh[b];
+            b = max(bin_of(mc, fe, lo_e, fscale), 0);
+            e = stab[b];
         }
-        const uint32_t k = fkey(v);
+        const uint32_t k = fkey(v), wl = __float_as_uint(e.z), wh = __float_as_uint(e.w);
         row[b] += inr ? (k < wl ? 0x10001u : 1u) : 0u;
         inside = inr && k >= wl && k <= wh;
         bo = b;
     };
     auto flush_rows = [&]() {                             // CTA-uniform
         __syncthreads();
-        for (int i = t; i < NB * 2; i += blockDim.x) {   // one thread per bin and field
-            const int bb = i >> 1, hi = i & 1;
-            unsigned int sum = 0;
-            for (int l = 0; l < 256; ++l) {
-                const unsigned int w = lc[l * kLaneRow + bb];
-                sum += hi ? w >> 16 : w & 0xffffu;
+        if (lane < NB) {                                 // lane = bin, each warp its own 32 rows
+            unsigned int vox = 0, below = 0;
+#pragma unroll 8
+            for (int l = t & ~31; l < (t & ~31) + 32; ++l) {
+                const unsigned int w = lc[l * kLaneRow + lane];
+                vox += w & 0xffffu;
+                below += w >> 16;
             }
-            if (sum) atomicAdd(&sc[3 * bb + (hi ? 0 : 2)], sum);
+            if (vox) atomicAdd(&sc[2 * lane], vox);
+            if (below) atomicAdd(&sc[2 * lane + 1], below);
         }
         __syncthreads();
         for (int i = 0; i < NB; ++i) row[i] = 0;
@@ -1315,103 +1103,31 @@ FY_D void k_bwin_count(const float* __restrict__ mean, const float* __restrict__
             }
     }
     wc.flush(cval, clab, &ctl->ncand, cap);
-    if (bad) s_bad = 1;
     flush_rows();
-    for (int i = t; i < NB * 3; i += blockDim.x)
-        if (sc[i]) atomicAdd(&ctl->bwc[i], (unsigned long long)sc[i]);
-    if (t == 0 && s_bad) atomicExch(&ctl->wfail, 1);
-}
-
-// After the counting pass: the bin counts, and, when the list fits and every bin's guess held,
-// the candidate block armed for the bins' digit passes with r = k - below for each bin of
-// >= 200 voxels (noise.c:123); otherwise the radix passes over the whole field (mode 1).
-// ctl->bwc per bin: [0] keys below the window, [2] the bin's voxels.
-FY_D void k_bwin_arm(NoiseCtl* __restrict__ ctl, NoiseCtl* __restrict__ cc, long long cap) {
-    fy_pdl_wait();
-    __shared__ int s_ok;
-    if (ctl->mode != kModeBinWin) {
-        if (threadIdx.x == 0) cc->mode = 3;
-        return;
-    }
-    const int t = threadIdx.x;
-    if (t == 0) s_ok = (long long)ctl->ncand <= cap && !ctl->wfail && !(noise_force_radix & 2);
-    __syncthreads();
-    long long cnt = 0, r = 0;
-    bool on = false;
     if (t < NB) {
-        const long long below = (long long)ctl->bwc[3 * t];
-        cnt = (long long)ctl->bwc[3 * t + 2];
-        on = cnt >= 200;
-        if (on) {
-            const double idx = ctl->flat_pct / 100.0 * (double)(cnt - 1);
-            r = (long long)idx - below;
-            if (r < 0) s_ok = 0;
-        }
+        if (sc[2 * t]) atomicAdd(&ctl->wvox[t], (unsigned long long)sc[2 * t]);
+        if (sc[2 * t + 1]) atomicAdd(&ctl->wbelow[t], (unsigned long long)sc[2 * t + 1]);
     }
-    __syncthreads();
-    if (!s_ok) {
-        if (t == 0) {
-            cc->mode = 3;
-            ctl->mode = 1;
-        }
-        return;
-    }
-    for (int i = t; i < NB * 256; i += blockDim.x) cc->hist[i] = 0;
-    if (t < NT_MAX) target_init(cc, t, on ? r : 0, 0, on);
-    if (t < NB) ctl->bcount[t] = (unsigned long long)cnt;
-    __syncthreads();
-    if (t == 0) {
-        cc->n = (long long)ctl->ncand;
-        cc->ntarget = NB;
-        cc->mode = 1;
-    }
-}
-
-// After the candidates' first digit pass (one block per bin): the bin's inside count is the sum
-// of its histogram; k and (when it exists) k+1 must be inside, else the bins go to the radix
-// passes over the whole field.
-FY_D void k_bwin_targets(NoiseCtl* __restrict__ ctl, NoiseCtl* __restrict__ cc) {
-    fy_pdl_wait();
-    __shared__ unsigned long long part[256];
-    if (cc->mode != 1 || ctl->mode != kModeBinWin) return;
-    const int b = vbx();
-    if (!cc->tactive[b]) return;
-    unsigned int* h = cc->hist + (size_t)b * 256;
-    part[threadIdx.x] = h[threadIdx.x];
-    __syncthreads();
-    for (int off = 128; off > 0; off >>= 1) {
-        if (threadIdx.x < off) part[threadIdx.x] += part[threadIdx.x + off];
-        __syncthreads();
-    }
-    const long long in = (long long)part[0];
-    const long long r = cc->trank[b];
-    const long long k = r + (long long)ctl->bwc[3 * b];
-    const bool has_next = k + 1 < (long long)ctl->bcount[b];
-    if (threadIdx.x == 0) {
-        if (r < in && (!has_next || r + 1 < in)) {
-            target_init(cc, b, r, in, true);
-        } else {
-            cc->mode = 3;
-            ctl->mode = 1;
-        }
-    }
-}
-
-// The bins' selected keys (k and k+1, in the form interp() reads) into the main block.
-FY_D void k_bwin_finish(NoiseCtl* __restrict__ ctl, const NoiseCtl* __restrict__ cc) {
-    fy_pdl_wait();
-    if (ctl->mode != kModeBinWin) return;
-    const int t = threadIdx.x;
+    if (!last_cta(ctl)) return;
+    // the targets: the flat_pct percentile of every bin of >= 200 voxels (noise.c:123), or of all
+    // variances when no bin has them (noise.c:166-171)
+    if (t >= 32) return;
+    long long cnt = 0;
     if (t < NB) {
-        ctl->tprefix[t] = cc->tprefix[t];
-        ctl->tnext[t] = cc->tneed_next[t] ? cc->tnext[t] : cc->tprefix[t];
-        ctl->tneed_next[t] = 1;
-        ctl->tactive[t] = cc->tactive[t];
+        cnt = (long long)__ldcg(&ctl->wvox[t]);
+        ctl->bcount[t] = (unsigned long long)cnt;
     }
-    __syncwarp();
+    const bool on = cnt >= 200, any = __any_sync(full, on);
+    if (t < NB) {
+        if (any) target_init(ctl, t, on ? (long long)(ctl->flat_pct / 100.0 * (double)(cnt - 1)) : 0, cnt, on);
+        else target_init(ctl, t, t == 0 ? (long long)(ctl->flat_pct / 100.0 * (double)(n - 1)) : 0, n, t == 0);
+    }
+    if (t < NB) window_buckets(ctl, t, kBinBuckets);
     if (t == 0) {
-        ctl->mode = kModeBinDone;
-        atomicOr(&noise_window_used, 2);
+        ctl->done_ctas = 0;
+        ctl->ntarget = any ? NB : 1;
+        ctl->mode = !any ? kVarField
+                         : ((long long)__ldcg(&ctl->ncand) > cap || (noise_force_radix & 2) ? kBinField : kBinWin);
     }
 }
 
@@ -1433,60 +1149,35 @@ FY_D double pct_small(double* v, int n, double pct) {       // percentile() on <
     return v[lo];
 }
 
-// stage 0: bin floors; arm the whole-volume fallback when no bin qualifies (mode 2).
-// stage 1: IRLS fit (FP64) and outputs.
-// One warp: lane b handles bin b's reads, so the bins' loads are in flight together; the
-// sequential fit then runs on lane 0 from shared memory.
-FY_D void k_noise_fit(NoiseCtl* ctl, int stage) {
+// IRLS fit (FP64) and outputs. One warp: lane b handles bin b, so the bins' loads are in flight
+// together. The used bins are compacted in bin order; the weights, residuals and the median of the
+// residuals are formed by one lane per bin, the five weighted sums by lane 0 in the reference's
+// order (noise.c:141-147), so every value equals the sequential fit's.
+FY_D void k_noise_fit(NoiseCtl* ctl) {
     fy_pdl_wait();
     static_assert(NB <= 32, "one lane per bin");
     const int lane = threadIdx.x;
-    if (stage == 0) {
-        bool use = false;
-        if (lane < NB) {
-            const long long c = (long long)ctl->bcount[lane];
-            if (c >= 200) {
-                const double idx = ctl->flat_pct / 100.0 * (double)(c - 1);
-                const long long k = (long long)idx;
-                ctl->bfloor[lane] = interp(ctl, lane, idx - (double)k, k + 1 < c);
-                use = true;
-            }
-        }
-        const int used = __popc(__ballot_sync(0xffffffffu, use));
-        if (lane != 0) return;
-        ctl->out_used = used;
-        if (used == 0) {                                  // noise.c:166-171
-            const long long n = ctl->n;
-            const double idx = ctl->flat_pct / 100.0 * (double)(n - 1);
-            for (int t = 0; t < NT_MAX; ++t) target_init(ctl, t, 0, 0, false);
-            target_init(ctl, 0, (long long)idx, n, true);
-            ctl->ntarget = 1;
-            ctl->mode = 2;
-        } else {
-            ctl->mode = 3;
-        }
-        return;
-    }
-    // stage 1: the used bins compacted in bin order; the weights, residuals and the median
-    // of the residuals are formed by one lane per bin, the five weighted sums by lane 0 in the
-    // reference's order (noise.c:141-147), so every value equals the sequential fit's
-    __shared__ double s_i[NB], s_f[NB], s_w[NB], s_r[NB];
+    __shared__ double s_i[NB], s_f[NB], s_w[NB], s_r[NB], s_one[NB];
     __shared__ long long s_c[NB];
     __shared__ double s_g, s_b;
     __shared__ int s_brk;
     const unsigned full = 0xffffffffu;
     const bool in_use = lane < NB && (long long)ctl->bcount[lane] >= 200;
+    if (lane < NB) s_one[lane] = 1.0;
     const unsigned um = __ballot_sync(full, in_use);
     const int used = __popc(um);
     if (in_use) {
         const int pos = __popc(um & ((1u << lane) - 1u));
         s_c[pos] = (long long)ctl->bcount[lane];
         s_i[pos] = 0.5 * (ctl->edge[lane] + ctl->edge[lane + 1]);
-        s_f[pos] = ctl->bfloor[lane];
+        const double idx = ctl->flat_pct / 100.0 * (double)(s_c[pos] - 1);
+        const long long k = (long long)idx;
+        s_f[pos] = interp(ctl, lane, idx - (double)k, k + 1 < s_c[pos]);     // the bin's floor
     }
     __syncwarp();
     double g = 0, bb = 0;
-    if (ctl->mode == 2) {
+    if (lane == 0) ctl->out_used = used;
+    if (ctl->mode == kVarField) {
         if (lane == 0) {
             const long long n = ctl->n;
             const double idx = ctl->flat_pct / 100.0 * (double)(n - 1);
@@ -1497,12 +1188,16 @@ FY_D void k_noise_fit(NoiseCtl* ctl, int stage) {
         if (lane < used) s_w[lane] = sqrt((double)s_c[lane]);
         __syncwarp();
         for (int it = 0; it < 4; it++) {
+            // the five weighted sums, one lane each, in the reference's order (noise.c:141-147):
+            // Sw += w, Swx += w*x, Swy += w*y, Swxx += w*x*x, Swxy += w*x*y (the factors that a sum
+            // lacks are 1; one lane doing all five took 7 us in all, lanes in five branches 27)
+            const double* f1 = lane == 0 ? s_one : (lane == 2 ? s_f : s_i);
+            const double* f2 = lane == 3 ? s_i : (lane == 4 ? s_f : s_one);
+            double acc = 0;
+            for (int i = 0; i < used; i++) acc += s_w[i] * f1[i] * f2[i];
+            const double Sw = __shfl_sync(full, acc, 0), Swx = __shfl_sync(full, acc, 1), Swy = __shfl_sync(full, acc, 2);
+            const double Swxx = __shfl_sync(full, acc, 3), Swxy = __shfl_sync(full, acc, 4);
             if (lane == 0) {
-                double Sw = 0, Swx = 0, Swy = 0, Swxx = 0, Swxy = 0;
-                for (int i = 0; i < used; i++) {
-                    const double wi = s_w[i], xi = s_i[i], yi = s_f[i];
-                    Sw += wi; Swx += wi * xi; Swy += wi * yi; Swxx += wi * xi * xi; Swxy += wi * xi * yi;
-                }
                 const double det = Sw * Swxx - Swx * Swx;
                 s_brk = fabs(det) < 1e-20;
                 if (!s_brk) {
@@ -1571,12 +1266,13 @@ unsigned grid_sel(long long n, int sms) {
 size_t fy_noise_ctl_bytes() { return (sizeof(NoiseCtl) + 255) & ~(size_t)255; }
 
 namespace {
-// Scratch layout (floats; every sub-array 256-byte aligned for the vector loads): mean, var,
-// bin labels (bytes), the candidates' control block, the sample of means, and the candidate
-// list (values, then labels) of capacity n/8 + 4096 (the window holds ~1% of the voxels).
+// Scratch layout (floats; every sub-array 256-byte aligned for the vector loads): mean, var, bin
+// labels (bytes; before the radix passes over the bins they hold the collected keys), the bins'
+// sample lists, and the candidate list (values, then labels) of capacity n/8 + 4096 (the windows
+// hold a few percent of the voxels).
 size_t round64(size_t v) { return (v + 63) & ~(size_t)63; }
 struct NoiseLayout {
-    size_t mean, var, bin, cc, samp, cval, clab, total;
+    size_t mean, var, bin, samp, cval, clab, total;
     long long cap;
 };
 NoiseLayout noise_layout(size_t n) {
@@ -1585,10 +1281,9 @@ NoiseLayout noise_layout(size_t n) {
     L.mean = 0;
     L.var = nr;
     L.bin = 2 * nr;
-    L.cc = L.bin + round64((n + 3) / 4);
-    L.samp = L.cc + round64((sizeof(NoiseCtl) + 3) / 4);
+    L.samp = L.bin + round64((n + 3) / 4);
     L.cap = (long long)((n + 7) / 8 + 4096);
-    L.cval = L.samp + (size_t)kSampleMax;
+    L.cval = L.samp + (size_t)NB * kBinListSmall;
     L.clab = L.cval + round64((size_t)L.cap);
     L.total = L.clab + round64(((size_t)L.cap + 3) / 4);
     return L;
@@ -1701,25 +1396,24 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
     float* mean = scratch + Lay.mean;
     float* var = scratch + Lay.var;
     uint8_t* bin = (uint8_t*)(scratch + Lay.bin);
-    NoiseCtl* cc = (NoiseCtl*)(scratch + Lay.cc);
-    float* sm = scratch + Lay.samp;
+    uint32_t* keys = (uint32_t*)(scratch + Lay.bin);
     float* cval = scratch + Lay.cval;
     uint8_t* clab = (uint8_t*)(scratch + Lay.clab);
     const int r = win / 2;
     const float inv_wc = (float)(1.0 / ((double)win * win * win));
     const unsigned g = grid_sel(n, sms), gc = grid_sel(Lay.cap, sms);
-    // passes that usually exit at once (the fallbacks, the k+1 scans): one CTA per SM, so the
-    // common case schedules few empty CTAs; when they do run, their grid-stride loops cover
+    // passes that usually exit at once (the radix passes): one CTA per SM, four for the bins', so
+    // the common case schedules few empty CTAs; when they do run, their grid-stride loops cover
     // every voxel
     const unsigned gs = (unsigned)(g < (unsigned)sms ? g : (unsigned)sms);
-    // candidate lists hold ~1-2% of the voxels (their capacity is n/8): two CTAs per SM
+    const unsigned gs4 = (unsigned)(g < 4u * (unsigned)sms ? g : 4u * (unsigned)sms);
+    // candidate lists hold a few percent of the voxels (their capacity is n/8): two CTAs per SM
     const unsigned gcl = (unsigned)(gc < 2u * (unsigned)sms ? gc : 2u * (unsigned)sms);
-    const size_t smem_all = 2 * 2048 * sizeof(unsigned int), smem_bin = NB * 256 * sizeof(unsigned int);
-    const size_t smem_bin_c = smem_bin + (size_t)(256 / 32) * kCompactBuf * (sizeof(float) + 1);
-    const size_t smem_keys = (kSampleMax + 256 * (kBoundThreads / 32)) * sizeof(uint32_t);   // keys + warp digit counts
-    const long long m = n < kSampleMax ? n : kSampleMax;
-    const unsigned long long wa = weyl_step((unsigned long long)n), wb = (unsigned long long)n / 3;
-    RUN(256, 1, k_noise_setup, 1, 256, 0, ctl, cc, n, flat_pct, ref_intensity);
+    const size_t smem_hist = kHist * sizeof(unsigned int);
+    const unsigned long long wa = weyl_step((unsigned long long)n);
+    // keys that a target can collect: the label region holds n/4 words
+    const long long lc_mean = n / 8 < kListMax ? n / 8 : kListMax, lc_bin = n / (4 * NB) < kListMax ? n / (4 * NB) : kListMax;
+    const size_t smem_stats = 2048 * sizeof(unsigned int);
     if (stats) {   // 1. stats
         fyzb::Params sp{};
         sp.nz = nz; sp.ny = ny; sp.nx = nx;
@@ -1730,90 +1424,33 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
         ++launches;
         if (!L.record) fy_prof_mark(st, "noise.stats");
     }
-    // 2a. 1st/99th percentile of the means: sample-guided window pass, then the radix passes
-    // of mode 1 over the candidates (control block cc, targets = labels); the radix passes
-    // over the whole field (11 + 11 + 10 bits, then the k+1 neighbours) run only if the
-    // window misses
-    RUN(256, 1, k_win_sample, 64, 256, 0, mean, ctl, sm, m, wa, wb);
-    RUN(kBoundThreads, 1, k_win_bounds, dim3(2, 2), kBoundThreads, smem_keys, sm, ctl, m);
+    // 2. the 1st/99th percentile of the means: window steps, then the radix passes behind them
+    RUN(kBoundThreads, 1, k_noise_begin, 1, kBoundThreads, 5 * smem_stats, mean, ctl, n, flat_pct, ref_intensity, wa,
+        (unsigned long long)n / 3, (wa * (unsigned long long)kBoundThreads) % (unsigned long long)n);
     RUN(256, 3, k_win_count, g, 256, 0, mean, ctl, cval, clab, Lay.cap);
-    RUN(32, 1, k_win_arm, 1, 1, 0, ctl, cc, Lay.cap);
-    for (int sh = 24; sh >= 0; sh -= 8) {
-        // the first digit's histogram sets the ranks (k_win_targets) before its scan; the
-        // later digits' scans run in each pass's last CTA
-        RUN(256, 1, (k_sel_hist<8, 1>), gcl, 256, smem_bin, nullptr, cval, clab, cc, sh, nullptr, nullptr, 0LL,
-            sh == 24 ? -1 : (sh == 0 ? 1 : 0));
-        if (sh == 24) {
-            RUN(256, 1, k_win_targets, 2, 256, 0, ctl, cc);
-            RUN(256, 1, k_sel_scan, 2, 256, 0, cc, 8, 1, 0);
-        }
-    }
-    RUN(256, 1, k_sel_next, gs, 256, 0, nullptr, cval, clab, cc, 1);
-    RUN(32, 1, k_win_finish, 1, 1, 0, ctl, cc);
-    const int all_digits[3][2] = {{21, 11}, {10, 11}, {0, 10}};
-    for (int i = 0; i < 3; ++i) {
-        if (all_digits[i][1] == 11) RUN(256, 1, (k_sel_hist<11, 0>), gs, 256, smem_all, mean, var, bin, ctl, all_digits[i][0], nullptr, nullptr, 0LL, i == 2 ? 1 : 0);
-        else RUN(256, 1, (k_sel_hist<10, 0>), gs, 256, smem_all, mean, var, bin, ctl, all_digits[i][0], nullptr, nullptr, 0LL, i == 2 ? 1 : 0);
-    }
-    RUN(256, 1, k_sel_next, gs, 256, 0, mean, var, bin, ctl, 0);
-    RUN(NT_MAX, 1, k_noise_bins_setup, 1, NT_MAX, 0, ctl);
+    RUN(512, 1, k_mean_bucket, gcl, 512, smem_hist, ctl, cval, clab, lc_mean);
+    RUN(256, 1, k_mean_collect, gcl, 256, 0, ctl, cval, clab, keys, lc_mean);
+    RUN(kBoundThreads, 1, k_cand_select, 2, kBoundThreads, 3 * smem_stats, ctl, keys, lc_mean, (int)kMeanWin, (int)kMeanCand, 1);
+    for (int sh = 24; sh >= 0; sh -= 8) RUN(256, 1, k_mean_radix, gs, 256, smem_hist, mean, ctl, cval, clab, sh);
     if (!L.record) fy_prof_mark(st, "noise.lohi");
-    // 2bw. per-bin flat_pct percentile of the variance through the bins' window: sample,
-    // bounds, one counting pass over mean and variance, then four digit passes over the
-    // candidates. The sample lives in the candidate region until the counting pass refills it.
+    // the per-bin flat_pct percentile of the variance, the same way. The sample lists use the
+    // candidate region when it is large enough (the counting pass refills it afterwards).
     {
         long long m2 = n < kBinSampleMax ? n : kBinSampleMax;
-        const long long m2cap = (Lay.cap - 64) * 4 / 5;    // keys, then labels 256-byte aligned
-        if (m2 > m2cap) m2 = m2cap;
-        uint32_t* skey = reinterpret_cast<uint32_t*>(cval);
-        uint8_t* slab = reinterpret_cast<uint8_t*>(cval + round64((size_t)m2));
-        RUN(256, 1, k_bwin_sample, 64, 256, 0, mean, var, ctl, skey, slab, m2, wa, (unsigned long long)n / 5);
-        RUN(kBoundThreads, 1, k_bwin_bounds, NB, kBoundThreads, smem_keys, skey, slab, ctl, m2);
+        const bool large = Lay.cap >= 2 * (long long)NB * kBinListSmall;
+        uint32_t* slist = large ? (uint32_t*)cval : (uint32_t*)(scratch + Lay.samp);
+        const int scap = !large ? kBinListSmall : (Lay.cap / NB < kBinListMax ? (int)(Lay.cap / NB) : kBinListMax);
+        RUN(kBinSampleThreads, 1, k_bin_sample, (unsigned)((m2 + kBinSampleThreads - 1) / kBinSampleThreads), kBinSampleThreads, 0,
+            mean, var, ctl, slist, scap, m2, wa, (unsigned long long)n / 5);
+        RUN(kBoundThreads, 1, k_bin_bounds, NB, kBoundThreads, 3 * smem_stats, slist, scap, ctl);
         RUN(256, 4, k_bwin_count, g, 256, 0, mean, var, ctl, cval, clab, Lay.cap);
-        RUN(256, 1, k_bwin_arm, 1, 256, 0, ctl, cc, Lay.cap);
-        for (int sh = 24; sh >= 0; sh -= 8) {
-            // the first digit's histogram gives the inside counts (k_bwin_targets) before its
-            // scan; the later digits' scans run in each pass's last CTA
-            RUN(256, 1, (k_sel_hist<8, 1>), gcl, 256, smem_bin, nullptr, cval, clab, cc, sh, nullptr, nullptr, 0LL,
-                sh == 24 ? -1 : (sh == 0 ? 1 : 0));
-            if (sh == 24) {
-                RUN(256, 1, k_bwin_targets, NB, 256, 0, ctl, cc);
-                RUN(256, 1, k_sel_scan, NB, 256, 0, cc, 8, 1, 0);
-            }
-        }
-        RUN(256, 1, k_sel_next, gcl, 256, 0, nullptr, cval, clab, cc, 1);
-        RUN(32, 1, k_bwin_finish, 1, 32, 0, ctl, cc);
+        RUN(512, 1, k_bin_bucket, gcl, 512, smem_hist, ctl, cval, clab, lc_bin);
+        RUN(256, 1, k_bin_collect, gcl, 256, 0, ctl, cval, clab, keys, lc_bin);
+        RUN(kBoundThreads, 1, k_cand_select, NB, kBoundThreads, 3 * smem_stats, ctl, keys, lc_bin, (int)kBinWin, (int)kBinCand, 2);
     }
-    // 2b. (when the bins' window missed) per-bin flat_pct percentile of the variance by radix
-    // passes over the whole field: 4 x 8 bits, then the k+1 neighbours;
-    // the first pass also labels the voxels with their bins and yields the bin counts. The
-    // third pass also lists the voxels that match their bin's 16-bit prefix (~1% of them),
-    // and the last digit runs over that list (falling back to the whole field if it overflows).
-    RUN(256, 1, (k_sel_hist<8, 1, true>), g, 256, smem_bin, mean, var, bin, ctl, 24, nullptr, nullptr, 0LL, -1);
-    RUN(256, 1, k_bin_targets, NB, 256, 0, ctl);
-    RUN(256, 1, k_sel_scan, NB, 256, 0, ctl, 8, 1, 0);
-    RUN(256, 1, (k_sel_hist<8, 1>), g, 256, smem_bin, mean, var, bin, ctl, 16, nullptr, nullptr, 0LL, 0);
-    RUN(32, 1, k_bin_cand_reset, 1, 1, 0, ctl);
-    RUN(256, 1, (k_sel_hist<8, 1, false, true>), g, 256, smem_bin_c, mean, var, bin, ctl, 8, cval, clab, Lay.cap, 0);
-    RUN(256, 1, k_bin_arm, 1, 256, 0, ctl, cc, Lay.cap);
-    RUN(256, 1, (k_sel_hist<8, 1>), gs, 256, smem_bin, mean, var, bin, ctl, 0, nullptr, nullptr, 0LL, 1);       // overflow only
-    RUN(256, 1, (k_sel_hist<8, 1>), gcl, 256, smem_bin, nullptr, cval, clab, cc, 0, nullptr, nullptr, 0LL, 1);  // the list
-    // k+1 past the selected key's 24-bit prefix: the list holds every key of the bin that shares
-    // its 16-bit prefix, so when it holds a larger key, its smallest larger key is the next one
-    // (a key in between would share the prefix and be listed too). Only targets whose next key
-    // leaves the 16-bit prefix are left to the whole-field scan below.
-    RUN(256, 1, k_sel_next, gcl, 256, 0, nullptr, cval, clab, cc, 1);
-    RUN(32, 1, k_bin_finish, 1, 1, 0, ctl, cc);
-    RUN(256, 1, k_sel_next, gs, 256, 0, mean, var, bin, ctl, 1);
-    RUN(32, 1, k_noise_fit, 1, 32, 0, ctl, 0);
+    for (int sh = 24; sh >= 0; sh -= 8) RUN(256, 1, k_bin_radix, gs4, 256, smem_hist, mean, var, bin, ctl, cval, clab, sh);
+    RUN(32, 1, k_noise_fit, 1, 32, 0, ctl);
     if (!L.record) fy_prof_mark(st, "noise.bin_select");
-    // 2c. fallback (mode 2 only): flat_pct percentile over all voxels' variance
-    for (int i = 0; i < 3; ++i) {
-        if (all_digits[i][1] == 11) RUN(256, 1, (k_sel_hist<11, 2>), gs, 256, smem_all, mean, var, bin, ctl, all_digits[i][0], nullptr, nullptr, 0LL, i == 2 ? 1 : 0);
-        else RUN(256, 1, (k_sel_hist<10, 2>), gs, 256, smem_all, mean, var, bin, ctl, all_digits[i][0], nullptr, nullptr, 0LL, i == 2 ? 1 : 0);
-    }
-    RUN(256, 1, k_sel_next, gs, 256, 0, mean, var, bin, ctl, 2);
-    RUN(32, 1, k_noise_fit, 1, 32, 0, ctl, 1);
     return cudaSuccess;
 }
 

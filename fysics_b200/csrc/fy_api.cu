@@ -284,7 +284,6 @@ int make_geom(int nz, int ny, int nx, SpecGeom& g, const char* what) {
                     g.px, FY_FFT_MAXN);
     g.hx = g.px / 2 + 1;
     g.hxp = (g.hx + 15) & ~15;
-    g.zero_pad = 0;
     return FY_OK;
 }
 

@@ -1,5 +1,5 @@
-// fy_deconv.cu -- the five deconvolution passes (fy_deconv.cuh) on the runtime plan, the
-// dispatch to the compile-time instantiations, and the Y pass shared with phase correlation.
+// fy_deconv.cu -- the five deconvolution passes (fy_deconv.cuh) on the runtime plan, and the
+// dispatch to the compile-time instantiations.
 #include "fy_deconv.cuh"
 
 namespace {
@@ -21,31 +21,6 @@ cudaError_t fy_launch_deconv(const DeconvLaunch& d, cudaStream_t st) {
         fy_prof_mark(st, kPassName[pass]);
     }
     return cudaSuccess;
-}
-
-// Y pass over `nplanes` stored planes of a half spectrum (shared with phase correlation):
-// sign -1 forward (rows >= ny gathered by reflection or zero), +1 inverse keeping rows
-// < keep_rows.
-cudaError_t fy_launch_spec_y(float2* spec, const SpecGeom& g, const FftPlan& ply, const float2* twy, int nplanes,
-                             int sign, int keep_rows, cudaStream_t st) {
-    const TileShape t = fy_tile_shape(g.py);
-    const size_t smem = (size_t)g.py * t.W * sizeof(float2) + (size_t)g.py * sizeof(float2);
-    dim3 grid(ceil_div_i(g.hx, t.W), nplanes);
-    return fy_with_e(t.E, [&](auto ec) -> cudaError_t {
-        constexpr int E = decltype(ec)::value;
-        if (sign < 0) {
-            auto k = k_y_fwd<0, E>;
-            cudaError_t e2 = fy_smem_optin(k, smem);
-            if (e2 != cudaSuccess) return e2;
-            k<<<grid, t.NT, smem, st>>>(spec, g, ply, twy, t.wlog);
-        } else {
-            auto k = k_y_inv<0, E>;
-            cudaError_t e2 = fy_smem_optin(k, smem);
-            if (e2 != cudaSuccess) return e2;
-            k<<<grid, t.NT, smem, st>>>(spec, g, ply, twy, keep_rows, t.wlog);
-        }
-        return cudaGetLastError();
-    });
 }
 
 // Expired bulk waits of the deconvolution's first pass in every unit that instantiates it.

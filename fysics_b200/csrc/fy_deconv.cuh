@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_x_fwd(const T* __restrict__ sr
         __syncthreads();
         for (int it = threadIdx.x; it < W * npad; it += blockDim.x) {
             const int l = dpad.div(it), x = g.nx + (it - l * npad);
-            s[l * LPX + x] = g.zero_pad ? make_float2(0.f, 0.f) : s[l * LPX + reflect_idx(x, g.nx)];
+            s[l * LPX + x] = s[l * LPX + reflect_idx(x, g.nx)];
         }
     }
     __syncthreads();
@@ -242,8 +242,8 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_y_fwd(float2* __restrict__ spe
     float2* col = spec + (size_t)blockIdx.y * g.py * g.hxp + blockIdx.x * W + ln.l;
     fft_line_pre<N, E, ct_pitch(N), -1>(s + ln.l, W, ln.tl, pl, stw,
                 [&](int i) {
-                    const int ys = i < g.ny ? i : (g.zero_pad ? -1 : reflect_idx(i, g.ny));
-                    return ys < 0 ? make_float2(0.f, 0.f) : col[(size_t)ys * g.hxp];
+                    const int ys = i < g.ny ? i : reflect_idx(i, g.ny);
+                    return col[(size_t)ys * g.hxp];
                 },
                 [&]() { load_twiddles(stw, tw, pl.n); },
                 [&](int i, float2 v) { col[(size_t)i * g.hxp] = v; });
@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_z_weight(float2* __restrict__ 
     __syncthreads();
     fft_line<N, E, ct_pitch(N), -1>(s + ln.l, W, ln.tl, pl, stw,
                 [&](int i) {
-                    const int zs = i < g.nz ? i : (g.zero_pad ? -1 : reflect_idx(i, g.nz));
-                    return zs < 0 ? make_float2(0.f, 0.f) : col[(size_t)zs * zstride];
+                    const int zs = i < g.nz ? i : reflect_idx(i, g.nz);
+                    return col[(size_t)zs * zstride];
                 },
                 [&](int z, float2 v) { s[z * W + ln.l] = v; });
     __syncthreads();

@@ -36,8 +36,6 @@ size_t fy_deconv_table_bytes(const SpecGeom& g);
 double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double param, int kind, double fz2s, void* host);
 int fy_deconv_setup(int nz, int ny, int nx, const fy_physics* p, double& param, int kind, double& fz2s,
                     double fmin, double fmax, DeconvLaunch& d, const char* what);
-cudaError_t fy_launch_spec_y(float2* spec, const SpecGeom& g, const FftPlan& ply, const float2* twy, int nplanes,
-                             int sign, int keep_rows, cudaStream_t st);
 cudaError_t fy_launch_cfft3d(float2* c, int nz, int ny, int nx, int nxp, int sign, cudaStream_t st);
 
 // Elementwise stream ops (stream.c)

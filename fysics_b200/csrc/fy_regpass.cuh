@@ -61,22 +61,20 @@ struct Column {
     }
 };
 
-// Points i >= n of an axis padded to N: the reflected point (paganin.c:121-128; N < 2n), or -1
-// where padding is zero.
-template <bool ZERO> FY_D int pad_src(int i, int n) { return i < n ? i : (ZERO ? -1 : 2 * n - 1 - i); }
+// Points i >= n of an axis padded to N are the reflected ones (paganin.c:121-128; N < 2n).
+FY_D int pad_src(int i, int n) { return i < n ? i : 2 * n - 1 - i; }
 
-template <int N, int PAD>     // PAD 0: every point stored; 1: reflect; 2: zero
+template <int N, bool PAD>
 FY_D void col_load(float2 (&v)[elems(N)], const float2* __restrict__ col, size_t es, int n, int t, bool valid) {
     const float2* p = col + (size_t)t * es;
     const size_t step = tpl(N) * es;
 #pragma unroll
     for (int m = 0; m < elems(N); ++m) {
-        if (PAD == 0) {
+        if (PAD) {
+            v[m] = valid ? col[(size_t)pad_src(t + tpl(N) * m, n) * es] : make_float2(0.f, 0.f);
+        } else {
             v[m] = valid ? *p : make_float2(0.f, 0.f);
             p += step;
-        } else {
-            const int src = pad_src<PAD == 2>(t + tpl(N) * m, n);
-            v[m] = valid && src >= 0 ? col[(size_t)src * es] : make_float2(0.f, 0.f);
         }
     }
 }
@@ -102,9 +100,9 @@ FY_D void col_fft(float2 (&v)[elems(N)], float2* __restrict__ s, int l, int t) {
     tail<N, SIGN>(v, t, s + C::tile);
 }
 
-// Y pass over the stored planes: forward (SIGN -1; rows >= nin gathered by PAD) or inverse,
+// Y pass over the stored planes: forward (SIGN -1; rows >= nin gathered by reflection) or inverse,
 // storing rows < nout.
-template <int N, int SIGN, int PAD>
+template <int N, int SIGN, bool PAD>
 __global__ void __launch_bounds__(Col<N>::NT, Col<N>::minb)
 k_col_y(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ ColTiles ct, const float2* __restrict__ tw, int nin,
         int nout) {
@@ -122,11 +120,11 @@ k_col_y(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ ColTiles 
     col_store<N>(v, col, g.hxp, nout, t, c.valid);
 }
 
-// Z pass: forward (planes >= nz gathered by PAD), radial LUT weight, inverse, planes < nz stored.
+// Z pass: forward (planes >= nz gathered by reflection), radial LUT weight, inverse, planes < nz stored.
 // The forward transform ends on the points where the inverse begins, so the weight is applied in
 // registers and the tile crosses shared memory twice in all (five times in the shared-memory
 // kernel, which also copied its tables to every tile).
-template <int N, int PAD>
+template <int N, bool PAD>
 __global__ void __launch_bounds__(Col<N>::NT, Col<N>::minb)
 k_col_z(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ ColTiles ct, const float2* __restrict__ tw,
         const float* lut, const double* fz2, const double* __restrict__ fy2, const double* __restrict__ fx2, double us) {
@@ -231,7 +229,7 @@ k_row_fwd(const T* __restrict__ src, float lo, float scale, float2* __restrict__
     float2 v[E];
 #pragma unroll
     for (int m = 0; m < E; ++m) {
-        const int i = t + TPL * m, x = PAD ? pad_src<false>(i, g.nx) : i;
+        const int i = t + TPL * m, x = PAD ? pad_src(i, g.nx) : i;
         float a = (float)__ldg(pa + x), b = (float)__ldg(pb + x);
         if (sizeof(T) == 1) {                             // fy_u8_to_phys, FMA as the reference build
             a = __fmaf_rn(a, scale, lo);
@@ -338,17 +336,16 @@ inline cudaError_t launch(K k, unsigned grid, int nt, size_t smem, cudaStream_t 
     return e != cudaSuccess ? e : fy_launch_pdl(k, dim3(grid), dim3(nt), smem, st, a...);
 }
 
-// A Y pass over `nplanes` stored planes; sign -1: rows >= ny gathered by the padding, every row
+// A Y pass over `nplanes` stored planes; sign -1: rows >= ny gathered by reflection, every row
 // stored; sign +1: rows < keep_rows stored.
 template <int N>
 inline cudaError_t launch_y(float2* spec, const SpecGeom& g, const float2* tw, int nplanes, int sign, int keep_rows,
                             cudaStream_t st) {
     using C = Col<N>;
     const ColTiles ct = col_tiles(g.hx, nplanes, C::W);
-    if (sign > 0) return launch(k_col_y<N, 1, 0>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, keep_rows);
-    if (g.ny == N) return launch(k_col_y<N, -1, 0>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, N);
-    if (g.zero_pad) return launch(k_col_y<N, -1, 2>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, g.ny, N);
-    return launch(k_col_y<N, -1, 1>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, g.ny, N);
+    if (sign > 0) return launch(k_col_y<N, 1, false>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, keep_rows);
+    if (g.ny == N) return launch(k_col_y<N, -1, false>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, N);
+    return launch(k_col_y<N, -1, true>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, g.ny, N);
 }
 
 // Pass `pass` (1..5) of a deconvolution whose axis length there is N.
@@ -373,8 +370,8 @@ cudaError_t deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
         using C = Col<N>;
         const ColTiles ct = col_tiles(g.hx, g.py, C::W);
         if (g.nz == N)
-            return launch(k_col_z<N, 0>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);
-        return launch(k_col_z<N, 1>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);
+            return launch(k_col_z<N, false>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);
+        return launch(k_col_z<N, true>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);
     }
     case 5: {
         const int nt = row_threads<N>(5);

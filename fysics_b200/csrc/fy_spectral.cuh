@@ -15,7 +15,6 @@ struct SpecGeom {
     int nz, ny, nx;   // logical volume
     int pz, py, px;   // padded transform sizes
     int hx, hxp;      // half-spectrum width and row pitch (complex elements)
-    int zero_pad;     // 0: reflect padding (paganin.c:121-128), 1: zero padding (phasecorr.c:76-87)
 };
 
 // Hermitian untangle of one two-for-one line: L = FFT(a + i b) ->

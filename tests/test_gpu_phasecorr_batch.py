@@ -19,7 +19,7 @@ def test_pairs_at_once(gpu, shape, pairs, window):
     rng = np.random.default_rng(sum(shape))
     f = rng.uniform(0, 1, (pairs, *shape)).astype(np.float32)
     m = np.stack([np.roll(f[i], (i, -i, 1), (0, 1, 2)) for i in range(pairs)])
-    m[-1] = 0.5                                              # a flat volume: degenerate, beside others that are not
+    f[-1] = m[-1] = 0.5                                      # flat volumes: degenerate, beside others that are not
     d_f, d_m = torch.from_numpy(f).cuda(), torch.from_numpy(m).cuda()
     scratch = torch.empty(lib.fy_gpu_phase_correlate_scratch_bytes(*shape), dtype=torch.uint8, device="cuda")
     sh, pk = (C.c_double * (3 * pairs))(), (C.c_double * pairs)()

@@ -11,8 +11,9 @@
 //   X phase one item = 4 output columns of one staged row: the row's values, the window
 //           sums of both quantities, two float4 stores; (TY + 2R) x TX/4 items (the halo
 //           rows included), one or two per thread.
-//   Y phase one thread = one output column x 4 output rows. Its (2R+1)-plane z ring of
-//           XY sums stays in registers and gives the box of plane zi - R to the epilogue.
+//   Y phase one thread = one output column x 4 output rows. Its XY sum of the plane is added to the
+//           2R windows open along z, kept in registers; the oldest is then complete and goes to the
+//           epilogue as the box of plane zi - R.
 // With TMA staging a plane takes one CTA barrier, between the X and Y phases: the X sums
 // alternate between two arrays, and each thread waits on the plane's mbarrier itself.
 // cp.async staging adds a barrier before the X phase (the copies of other threads).
@@ -72,6 +73,9 @@ struct Params {
     int wci;               // NOISE: win^3
     int out_mode;
     int nz, ny, nx, zchunk;
+    // voxels per row of f0, of the guide, of o0/o1 and of o2: nx, or for a field of the library's own
+    // nx rounded up to 4 voxels, so that its rows are 16-byte aligned for TMA staging (fy_pitch)
+    int pf0, pg, po, pmv;
     RingApply ra;          // GUIDED_OUT, out_mode 0: ring subtraction on the output (optional)
 };
 
@@ -84,9 +88,9 @@ struct Geo {
     static constexpr int STAGE = (SY * RW + 31) / 32 * 32;      // floats per staged plane (128 B multiple)
     static constexpr int XS = SY * TX;                          // float2 per X-sum array
     static constexpr int GUIDE = C == 2 ? TX * TY : 0;           // floats per staged guide tile
-    // the staged planes, the guide tiles (output passes), two X-sum arrays (alternate planes),
-    // the reciprocal counts, 128 B for alignment
-    static constexpr size_t bytes = (size_t)(NS * (STAGE + GUIDE) + 4 * XS + TX + TY) * sizeof(float) + 128;
+    // the staged planes, the guide tiles (output passes), two X-sum arrays (alternate planes), 128 B
+    // for alignment
+    static constexpr size_t bytes = (size_t)(NS * (STAGE + GUIDE) + 4 * XS) * sizeof(float) + 128;
 };
 
 FY_D float recip_count(int p, int L, int r) {
@@ -102,7 +106,7 @@ FY_D float2 mul2(float2 a, float f) { return __fmul2_rn(a, make_float2(f, f)); }
 // reciprocal in-bounds counts (guided.c:121-128).
 FY_D float2 guided_mv(float2 sums, float rxyz, float c) {
     const float2 e = mul2(sums, rxyz);                 // E[I-c], E[(I-c)^2]
-    float var = e.y - e.x * e.x;
+    float var = __fmaf_rn(-e.x, e.x, e.y);
     if (var < 0.f) var = 0.f;
     return make_float2(e.x + c, var);
 }
@@ -111,7 +115,7 @@ FY_D float2 guided_mv(float2 sums, float rxyz, float c) {
 // output pass from (mean, var) share it, so both forms of the filter agree bit for bit.
 FY_D float2 guided_ab(float2 mv, float eps) {
     const float a = __fdividef(mv.y, mv.y + eps);
-    return make_float2(a, mv.x * (1.0f - a));
+    return make_float2(a, __fmul_rn(mv.x, 1.0f - a));
 }
 
 FY_D void cp16(float* sdst, const float* gsrc, bool valid) {
@@ -199,21 +203,21 @@ template <int R, int C, bool VEC>
 FY_D void stage_plane(float* dst, const Params& p, int zi, int x0, int y0) {
     using G = Geo<R, C>;
     const bool zin = zi >= 0 && zi < p.nz;
-    const size_t pbase = (size_t)(zin ? zi : 0) * p.ny * p.nx;
+    const size_t pbase = (size_t)(zin ? zi : 0) * p.ny * p.pf0;
     if (VEC) {
         constexpr int Q = G::RW / 4;
         for (int k = threadIdx.x; k < G::SY * Q; k += NT) {
             const int yy = k / Q, q = k - yy * Q;
             const int gy = y0 - R + yy, gx = x0 - 4 + 4 * q / C;
             const bool ok = zin && gy >= 0 && gy < p.ny && gx >= 0 && gx < p.nx;
-            cp16(dst + yy * G::RW + 4 * q, ok ? p.f0 + (pbase + (size_t)gy * p.nx + gx) * C : p.f0, ok);
+            cp16(dst + yy * G::RW + 4 * q, ok ? p.f0 + (pbase + (size_t)gy * p.pf0 + gx) * C : p.f0, ok);
         }
     } else {
         for (int k = threadIdx.x; k < G::SY * G::RW; k += NT) {
             const int yy = k / G::RW, e = k - yy * G::RW;
             const int gy = y0 - R + yy, gx = x0 - 4 + e / C;
             const bool ok = zin && gy >= 0 && gy < p.ny && gx >= 0 && gx < p.nx;
-            cp4(dst + k, ok ? p.f0 + (pbase + (size_t)gy * p.nx + gx) * C + (e - (e / C) * C) : p.f0, ok);
+            cp4(dst + k, ok ? p.f0 + (pbase + (size_t)gy * p.pf0 + gx) * C + (e - (e / C) * C) : p.f0, ok);
         }
     }
 }
@@ -221,29 +225,32 @@ FY_D void stage_plane(float* dst, const Params& p, int zi, int x0, int y0) {
 // One CTA's tile (bx, by) and z chunk bz of a box pass. Returns false when a bounded wait gave
 // up (the CTA then raised zb_timeout and drained its copies). With TMA it leaves the slot
 // barriers invalidated, so the CTA can run another tile.
+//
+// What depends on the tile's place (columns and rows outside the volume, in-bounds counts) is a
+// constant of each thread, formed once before the plane loop: the shift of each of its taps (0
+// outside), its reciprocal counts, its outputs' offsets. The loop then tests nothing per voxel but
+// the output rows, and has one form for inner and edge tiles. Measured at 512^3, statistics / guided
+// output: tests in the loop, unrolled 2R+1 times for a z ring of plane sums, 627 / 720 us; a second,
+// test-free form for inner tiles beside it, slower (two long loops share the instruction cache);
+// this form 543 / 658 us.
 template <int R, int KIND, bool VEC, bool TMA>
 FY_D bool zbox_tile(const Params& p, const TmaRef& tm, int bx, int by, int bz, unsigned long long* bars) {
     constexpr int C = out_kind(KIND) ? 2 : 1;
     using G = Geo<R, C>;
     constexpr int NR = G::NR;
+    using Off = typename std::conditional<TMA, unsigned, size_t>::type;   // TMA: nx < 2^24 (launch_r)
     extern __shared__ float4 zb_smem4[];
     float* stage = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(zb_smem4) + 127) & ~(uintptr_t)127);
     float* sguide = stage + NS * G::STAGE;                         // NS guide tiles (output passes)
     float2* xs = reinterpret_cast<float2*>(sguide + NS * G::GUIDE);  // X sums of both quantities, 2 x [SY][TX]
-    float* rx = reinterpret_cast<float*>(xs + 2 * G::XS);
-    float* ry = rx + TX;
     const int t = threadIdx.x;
     const int nz = p.nz, ny = p.ny, nx = p.nx;
     const int x0 = bx * TX, y0 = by * TY;
     const int zs = bz * p.zchunk, ze = min(nz, zs + p.zchunk);
-    const size_t plane = (size_t)ny * nx;
     // per-tile shift: one constant for every window this CTA forms
-    const float c = out_kind(KIND) ? 0.f : __ldg(p.f0 + (size_t)zs * plane + (size_t)y0 * nx + x0);
+    const float c = out_kind(KIND) ? 0.f : __ldg(p.f0 + ((size_t)zs * ny + y0) * p.pf0 + x0);
     float eps = p.eps;
     if ((KIND == ZB_GUIDED_AB || KIND == ZB_GUIDED_OUT_MV) && p.eps_ptr) eps = *p.eps_ptr;   // device noise model
-    if (t < TX) rx[t] = x0 + t < nx ? recip_count(x0 + t, nx, R) : 0.f;
-    if (t < TY) ry[t] = y0 + t < ny ? recip_count(y0 + t, ny, R) : 0.f;
-    const bool cols_in = x0 - 4 >= 0 && x0 + TX + 4 <= nx;       // no column of the staged rows is outside
     const int zfirst = zs - R, zend = ze + R;
     int zissued = min(zfirst + NS - 2, zend - 1);                // thread 0: last plane whose copy it issued
     const int first_polls = TMA ? zb_first_wait_polls : 0;
@@ -270,15 +277,49 @@ FY_D bool zbox_tile(const Params& p, const TmaRef& tm, int bx, int by, int bz, u
             cp_commit();
         }
     }
+    // X-phase role: a 4-column item, and for the first threads a 2-column one (half of a 4-column item
+    // of the 2R halo rows left over), so the phase that gates the plane's barrier costs 1.5 item times
+    // instead of 2. Taps: the shift of each of the item's columns, 0 outside the volume (staged as 0);
+    // reciprocal in-bounds counts of its output columns.
+    constexpr int NITEM = G::SY * (TX / 4), NHALF = 2 * (NITEM - NT);
+    static_assert(NITEM >= NT && NHALF <= NT, "one full and at most one half item per thread");
+    const int ya = t >> 4, xa = (t & 15) << 2;
+    const int yb = (NT + (t >> 1)) >> 4, xb = (((NT + (t >> 1)) & 15) << 2) + 2 * (t & 1);
+    float ca[4 + 2 * R], cb[2 + 2 * R], rxa[4], rxb[2];
+    if (!out_kind(KIND)) {
+#pragma unroll
+        for (int j = 0; j < 4 + 2 * R; ++j) {
+            const int gy = y0 - R + ya, gxj = x0 + xa - R + j;
+            ca[j] = gy >= 0 && gy < ny && gxj >= 0 && gxj < nx ? c : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 2 + 2 * R; ++j) {
+            const int gy = y0 - R + yb, gxj = x0 + xb - R + j;
+            cb[j] = gy >= 0 && gy < ny && gxj >= 0 && gxj < nx ? c : 0.f;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) rxa[k] = x0 + xa + k < nx ? recip_count(x0 + xa + k, nx, R) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) rxb[k] = x0 + xb + k < nx ? recip_count(x0 + xb + k, nx, R) : 0.f;
+    }
     // Y-phase role: output column xc, output rows 4*rg .. 4*rg+3
     const int xc = t & (TX - 1), rg = t >> 6;
     const int gx = x0 + xc;
-    int cyx[4];                                                   // NOISE: in-bounds XY window size
+    const int rows = gx < nx ? min(4, ny - y0 - 4 * rg) : 0;     // this thread's output rows (may be < 0)
+    float ryk[4], nxy[4];                                         // OUT: 1/count_y; else 1/count_x/count_y, and NOISE the count
+    Off off[4];                                                   // outputs: elements from the tile's first voxel
+    Off goff[4];                                                  // the guide's, where it is not staged
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         const int gy = y0 + 4 * rg + k;
-        cyx[k] = (min(gy + R, ny - 1) - max(gy - R, 0) + 1) * (min(gx + R, nx - 1) - max(gx - R, 0) + 1);
+        const float ry = gy < ny ? recip_count(gy, ny, R) : 0.f;
+        ryk[k] = out_kind(KIND) ? ry : (gx < nx ? recip_count(gx, nx, R) : 0.f) * ry;
+        nxy[k] = (float)((min(gy + R, ny - 1) - max(gy - R, 0) + 1) * (min(gx + R, nx - 1) - max(gx - R, 0) + 1));
+        off[k] = (Off)(4 * rg + k) * (Off)p.po + (Off)xc;
+        goff[k] = (Off)(4 * rg + k) * (Off)p.pg + (Off)xc;
     }
+    const float wcf = (float)p.wci;
     // GUIDED_OUT: ring radius of this thread's 4 output voxels (dering.c:200-248)
     bool rings = false;
     int ri[4] = {0, 0, 0, 0};
@@ -295,218 +336,200 @@ FY_D bool zbox_tile(const Params& p, const TmaRef& tm, int bx, int by, int bz, u
             ri[k] = (int)(sqrt(gyd * gyd + gxd * gxd) + 0.5);
         }
     }
-    float2 rz2[NR][4];                                            // z ring of XY sums
+    float2 acc[2 * R][4];           // the windows begun 2R, ..., 1 planes ago: their sums so far
 #pragma unroll
-    for (int q = 0; q < NR; ++q)
+    for (int q = 0; q < 2 * R; ++q)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) rz2[q][k] = make_float2(0.f, 0.f);
+        for (int k = 0; k < 4; ++k) acc[q][k] = make_float2(0.f, 0.f);
 
-    // The plane loop is unrolled by NR so the z ring rotates by naming: plane zi lands in
-    // ring slot ph = (zi - zfirst) mod NR, and the window of plane zi - R is slots ph+1 ..
-    // ph+NR (mod NR) in ascending z.
-    for (int zi0 = zfirst; zi0 < zend; zi0 += NR) {
+    for (int zi = zfirst; zi < zend; ++zi) {
+        const int it = zi - zfirst, slot = it & (NS - 1);
+        // TMA: no barrier before the X phase. Every thread passed the previous plane's
+        // barrier, so plane zi - 1's slot is read out (thread 0 refills it) and the X sums
+        // of plane zi - 2, which share this plane's array, are read out.
+        bool ok = true;
+        float2* xcur = xs;
+        if (TMA) {
+            ok = mbar_wait_bounded(&bars[slot], (unsigned)((it / NS) & 1), it == 0 ? first_polls : kWaitSpins);
+            xcur = xs + (it & 1) * G::XS;
+        } else {
+            cp_wait<NS - 2>();
+            __syncthreads();             // plane zi landed for every thread; xs free again
+            const int zn = zi + NS - 1;
+            if (zn < zend) stage_plane<R, C, VEC>(stage + ((zn - zfirst) & (NS - 1)) * G::STAGE, p, zn, x0, y0);
+            cp_commit();
+        }
+        const int zo = zi - R;
+        const bool emit = zo >= zs && zo < ze;
+        float gv[4] = {0.f, 0.f, 0.f, 0.f};
+        if (out_kind(KIND) && p.out_mode == 0 && emit && !gstage) {   // issued early, used after the Y phase
+            const float* gb = p.guide + ((size_t)zo * ny + y0) * p.pg + x0;
 #pragma unroll
-        for (int ph = 0; ph < NR; ++ph) {
-            const int zi = zi0 + ph;
-            if (zi >= zend) break;
-            const int slot = (zi - zfirst) & (NS - 1);
-            // TMA: no barrier before the X phase. Every thread passed the previous plane's
-            // barrier, so plane zi - 1's slot is read out (thread 0 refills it) and the X sums
-            // of plane zi - 2, which share this plane's array, are read out.
-            bool ok = true;
-            float2* xcur = xs;
-            if (TMA) {
-                ok = mbar_wait_bounded(&bars[slot], (unsigned)(((zi - zfirst) / NS) & 1),
-                                       zi == zfirst ? first_polls : kWaitSpins);
-                xcur = xs + ((zi - zfirst) & 1) * G::XS;
-            } else {
-                cp_wait<NS - 2>();
-                __syncthreads();             // plane zi landed for every thread; xs free again
-                const int zn = zi + NS - 1;
-                if (zn < zend) stage_plane<R, C, VEC>(stage + ((zn - zfirst) & (NS - 1)) * G::STAGE, p, zn, x0, y0);
-                cp_commit();
-            }
-            const int zo = zi - R;
-            const bool emit = zo >= zs && zo < ze && gx < nx;
-            const size_t obase = (size_t)(emit ? zo : 0) * plane + (size_t)(y0 + 4 * rg) * nx + gx;
-            float gv[4] = {0.f, 0.f, 0.f, 0.f};
-            if (out_kind(KIND) && p.out_mode == 0 && emit && !gstage) {   // issued early, used after the Y phase
+            for (int k = 0; k < 4; ++k)
+                if (k < rows) gv[k] = __ldg(gb + goff[k]);
+        }
+        const float* sp = stage + slot * G::STAGE;
+        const float zf = zi >= 0 && zi < nz ? 1.f : 0.f;              // outside planes: no shift
+        // X phase: an item is IW output columns of one staged row starting at column xi; P[j] = both
+        // quantities of column xi - R + j.
+        auto xitem = [&](auto wc, int yy, int xi, const float* cj, const float* rxk) {
+            constexpr int IW = decltype(wc)::value, NP = IW + 2 * R;
+            float2 P[NP + 2];
+            if (C == 2) {                    // interleaved pairs: float4 = two columns
+                constexpr int J0 = (4 - R) & ~1;                      // first column read, even
+                const float* row = sp + yy * G::RW + 2 * (xi + J0);
+                float2 q[NP + 2];
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (y0 + 4 * rg + k < ny) gv[k] = __ldg(p.guide + obase + (size_t)k * nx);
-            }
-            const float* sp = stage + slot * G::STAGE;
-            const bool zin = zi >= 0 && zi < nz;
-            // X phase, every staged row (the TY output rows and the 2R halo rows): an item is IW
-            // output columns of one row starting at xs, P[j] = both quantities of staged column
-            // x0 - 4 + xs + j. Each thread takes one 4-column item; the 2R halo rows' 4-column
-            // items left over are split into 2-column halves spread over the first threads, so
-            // the phase that gates the plane's barrier costs 1.5 item times instead of 2.
-            // (One-column items for the halo rows cost (2R+1) taps' conversions per output
-            // instead of (4+2R)/4; every split keeps the same taps in the same order.)
-            auto xitem = [&](auto wc, int yy, int xs) {
-                constexpr int IW = decltype(wc)::value;
-                float2 P[12];
-                if (C == 2) {                    // interleaved pairs: float4 = two columns
-                    const float* row = sp + yy * G::RW + 2 * xs;
-#pragma unroll
-                    for (int j2 = (4 - R) / 2; j2 <= (IW + 3 + R) / 2; ++j2) {
-                        const float4 v = *reinterpret_cast<const float4*>(row + 4 * j2);
-                        P[2 * j2] = make_float2(v.x, v.y);
-                        P[2 * j2 + 1] = make_float2(v.z, v.w);
-                    }
-                    if (KIND == ZB_GUIDED_OUT_MV) {          // (mean, var) -> (a, b)
-#pragma unroll
-                        for (int j = 4 - R; j < IW + 4 + R; ++j) P[j] = guided_ab(P[j], eps);
-                    }
-                } else {
-                    const float* row = sp + yy * G::RW + xs;
-                    float q1[12];
-                    if (IW == 4) {                   // xs a multiple of 4: 16-byte loads
-#pragma unroll
-                        for (int j = 0; j < 3; ++j) {
-                            const float4 v = *reinterpret_cast<const float4*>(row + 4 * j);
-                            q1[4 * j] = v.x; q1[4 * j + 1] = v.y; q1[4 * j + 2] = v.z; q1[4 * j + 3] = v.w;
-                        }
-                    } else {                         // xs even: 8-byte loads
-#pragma unroll
-                        for (int j = (4 - R) & ~1; j < IW + 4 + R; j += 2) {
-                            const float2 v = *reinterpret_cast<const float2*>(row + j);
-                            q1[j] = v.x; q1[j + 1] = v.y;
-                        }
-                    }
-                    const int gy = y0 - R + yy;
-                    const bool rin = zin && gy >= 0 && gy < ny;
-                    if (cols_in) {
-                        const float cs = rin ? c : 0.f;           // outside rows were staged as 0
-#pragma unroll
-                        for (int j = 4 - R; j < IW + 4 + R; ++j) q1[j] = q1[j] - cs;
-                    } else {
-#pragma unroll
-                        for (int j = 4 - R; j < IW + 4 + R; ++j) {
-                            const int gxj = x0 - 4 + xs + j;
-                            q1[j] = (rin && gxj >= 0 && gxj < nx) ? q1[j] - c : 0.f;
-                        }
-                    }
-#pragma unroll
-                    for (int j = 4 - R; j < IW + 4 + R; ++j) P[j] = make_float2(q1[j], q1[j] * q1[j]);
+                for (int j = 0; j < NP + (4 - R - J0); j += 2) {
+                    const float4 v = *reinterpret_cast<const float4*>(row + 2 * j);
+                    q[j] = make_float2(v.x, v.y);
+                    q[j + 1] = make_float2(v.z, v.w);
                 }
-                float2 o[IW];
 #pragma unroll
-                for (int k = 0; k < IW; ++k) {
-                    float2 sm = P[4 + k - R];
-#pragma unroll
-                    for (int j = 5 + k - R; j <= 4 + k + R; ++j) sm = add2(sm, P[j]);
-                    if (out_kind(KIND)) sm = mul2(sm, rx[xs + k]);
-                    o[k] = sm;
-                }
-                float4* dst = reinterpret_cast<float4*>(xcur + yy * TX + xs);
-#pragma unroll
-                for (int k2 = 0; k2 < IW / 2; ++k2) dst[k2] = make_float4(o[2 * k2].x, o[2 * k2].y, o[2 * k2 + 1].x, o[2 * k2 + 1].y);
-            };
-            constexpr int NITEM = G::SY * (TX / 4), NHALF = 2 * (NITEM - NT);
-            static_assert(NITEM >= NT && NHALF <= NT, "one full and at most one half item per thread");
-            xitem(std::integral_constant<int, 4>{}, t >> 4, (t & 15) << 2);
-            if (t < NHALF) {
-                const int it = NT + (t >> 1);
-                xitem(std::integral_constant<int, 2>{}, it >> 4, ((it & 15) << 2) + 2 * (t & 1));
-            }
-            if (TMA) {
-                if (__syncthreads_or(!ok)) {      // plane zi never landed: flag, drain, return
-                    if (t == 0) {
-                        atomicExch(&zb_timeout, 1);
-                        for (int zq = zi; zq <= zissued; ++zq)          // loads issued so far
-                            mbar_wait_bounded(&bars[(zq - zfirst) & (NS - 1)], (unsigned)(((zq - zfirst) / NS) & 1));
-                    }
-                    __syncthreads();
-                    return false;
-                }
-                // Refill the slot of plane zi - 1: past this barrier every thread has finished
-                // plane zi - 1, its staged rows and its guide tile alike.
-                const int zn = zi + NS - 1;
-                if (t == 0 && zn < zend) {
-                    const int sn = (zn - zfirst) & (NS - 1);
-                    tma_stage<R, C>(stage + sn * G::STAGE, guide_slot(sn, zn), tm, &bars[sn], zn, x0, y0);
-                    zissued = zn;
+                for (int j = 0; j < NP; ++j) {
+                    P[j] = q[j + (4 - R - J0)];
+                    if (KIND == ZB_GUIDED_OUT_MV) P[j] = guided_ab(P[j], eps);     // (mean, var) -> (a, b)
                 }
             } else {
+                float q1[12];
+                const float* row = sp + yy * G::RW + xi;
+                if (IW == 4) {                   // xi a multiple of 4: 16-byte loads
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) {
+                        const float4 v = *reinterpret_cast<const float4*>(row + 4 * j);
+                        q1[4 * j] = v.x; q1[4 * j + 1] = v.y; q1[4 * j + 2] = v.z; q1[4 * j + 3] = v.w;
+                    }
+                } else {                         // xi even: 8-byte loads
+#pragma unroll
+                    for (int j = (4 - R) & ~1; j < IW + 4 + R; j += 2) {
+                        const float2 v = *reinterpret_cast<const float2*>(row + j);
+                        q1[j] = v.x; q1[j + 1] = v.y;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < NP; ++j) {
+                    const float u = __fmaf_rn(-cj[j], zf, q1[4 - R + j]);
+                    P[j] = make_float2(u, __fmul_rn(u, u));
+                }
+            }
+            float2 o[IW];
+#pragma unroll
+            for (int k = 0; k < IW; ++k) {
+                float2 sm = P[k];
+#pragma unroll
+                for (int j = 1; j <= 2 * R; ++j) sm = add2(sm, P[k + j]);
+                if (out_kind(KIND)) sm = mul2(sm, rxk[k]);
+                o[k] = sm;
+            }
+            float4* dst = reinterpret_cast<float4*>(xcur + yy * TX + xi);
+#pragma unroll
+            for (int k2 = 0; k2 < IW / 2; ++k2) dst[k2] = make_float4(o[2 * k2].x, o[2 * k2].y, o[2 * k2 + 1].x, o[2 * k2 + 1].y);
+        };
+        xitem(std::integral_constant<int, 4>{}, ya, xa, ca, rxa);
+        if (t < NHALF) xitem(std::integral_constant<int, 2>{}, yb, xb, cb, rxb);
+        if (TMA) {
+            if (__syncthreads_or(!ok)) {      // plane zi never landed: flag, drain, return
+                if (t == 0) {
+                    atomicExch(&zb_timeout, 1);
+                    for (int zq = zi; zq <= zissued; ++zq)          // loads issued so far
+                        mbar_wait_bounded(&bars[(zq - zfirst) & (NS - 1)], (unsigned)(((zq - zfirst) / NS) & 1));
+                }
                 __syncthreads();
+                return false;
             }
-            // Y phase -> ring slot ph
-            {
-                float2 a[4 + 2 * R];
-#pragma unroll
-                for (int j = 0; j < 4 + 2 * R; ++j) a[j] = xcur[(4 * rg + j) * TX + xc];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float2 sm = a[k];
-#pragma unroll
-                    for (int j = 1; j <= 2 * R; ++j) sm = add2(sm, a[k + j]);
-                    if (out_kind(KIND)) sm = mul2(sm, ry[4 * rg + k]);
-                    rz2[ph][k] = sm;
-                }
+            // Refill the slot of plane zi - 1: past this barrier every thread has finished
+            // plane zi - 1, its staged rows and its guide tile alike.
+            const int zn = zi + NS - 1;
+            if (t == 0 && zn < zend) {
+                const int sn = (zn - zfirst) & (NS - 1);
+                tma_stage<R, C>(stage + sn * G::STAGE, guide_slot(sn, zn), tm, &bars[sn], zn, x0, y0);
+                zissued = zn;
             }
-            if (!emit) continue;
-            if (out_kind(KIND) && rings) {                        // this plane's ring slab (dering.c:212-215)
-                const long zg = p.ra.z0 + zo;
-                if (!(zg >= rlo && zg < rhi)) {                   // left the cached slab's planes: divide once
-                    const long q = zg / p.ra.slab_z;
-                    rlo = q * p.ra.slab_z;
-                    rhi = rlo + p.ra.slab_z;
-                    long sl = q;
-                    if (sl < 0) sl = 0;
-                    if (sl >= p.ra.nslab) sl = p.ra.nslab - 1;
-                    if (sl != rslab) {
-                        rslab = sl;
+        } else {
+            __syncthreads();
+        }
+        // Y phase: each XY sum of the plane is added to the open windows, which move up by one: every
+        // window is summed in ascending z from its first plane, and the oldest is complete
+        float2 win[4];
+        {
+            float2 a[4 + 2 * R];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            rv[k] = ri[k] < p.ra.nr ? __ldg(p.ra.ring + (size_t)sl * p.ra.nr + ri[k]) : 0.f;
-                    }
-                }
-            }
-            const bool zint = zo >= R && zo + R <= nz - 1;        // the window's planes all inside
-            const float rz = zint ? rz_in : recip_count(zo, nz, R);
-            const int cz = zint ? 2 * R + 1 : min(zo + R, nz - 1) - max(zo - R, 0) + 1;
+            for (int j = 0; j < 4 + 2 * R; ++j) a[j] = xcur[(4 * rg + j) * TX + xc];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                if (y0 + 4 * rg + k >= ny) continue;
-                float2 sm = rz2[(ph + 1) % NR][k];
+                float2 sm = a[k];
 #pragma unroll
-                for (int q = 2; q <= NR; ++q) sm = add2(sm, rz2[(ph + q) % NR][k]);
-                const float s1 = sm.x, s2 = sm.y;
-                const size_t o = obase + (size_t)k * nx;
-                if (KIND == ZB_NOISE) {
-                    const int nini = cz * cyx[k];
-                    const float nin = (float)nini;
-                    // raw sums: S1 = S1' + nin*c, S2 = S2' + 2c*S1' + nin*c^2
-                    const float m = (s1 + nin * c) * p.inv_wc;
-                    float v;
-                    if (nini == p.wci) {                           // interior: shifted, cancellation-free
-                        const float e1 = s1 * p.inv_wc;
-                        v = s2 * p.inv_wc - e1 * e1;
-                    } else {
-                        v = (s2 + 2.0f * c * s1 + nin * c * c) * p.inv_wc - m * m;
-                    }
-                    if (v < 0.f) v = 0.f;
-                    p.o0[o] = m;
-                    p.o1[o] = v;
-                    if (p.o2)
-                        reinterpret_cast<float2*>(p.o2)[o] = guided_mv(sm, rx[xc] * ry[4 * rg + k] * rz, c);
-                } else if (KIND == ZB_GUIDED_AB) {
-                    reinterpret_cast<float2*>(p.o0)[o] = guided_ab(guided_mv(sm, rx[xc] * ry[4 * rg + k] * rz, c), eps);
+                for (int j = 1; j <= 2 * R; ++j) sm = add2(sm, a[k + j]);
+                if (out_kind(KIND)) sm = mul2(sm, ryk[k]);
+                win[k] = add2(acc[0][k], sm);
+#pragma unroll
+                for (int q = 0; q + 1 < 2 * R; ++q) acc[q][k] = add2(acc[q + 1][k], sm);
+                acc[2 * R - 1][k] = sm;
+            }
+        }
+        if (!emit) continue;
+        if (out_kind(KIND) && rings) {                        // this plane's ring slab (dering.c:212-215)
+            const long zg = p.ra.z0 + zo;
+            if (!(zg >= rlo && zg < rhi)) {                   // left the cached slab's planes: divide once
+                const long q = zg / p.ra.slab_z;
+                rlo = q * p.ra.slab_z;
+                rhi = rlo + p.ra.slab_z;
+                long sl = q;
+                if (sl < 0) sl = 0;
+                if (sl >= p.ra.nslab) sl = p.ra.nslab - 1;
+                if (sl != rslab) {
+                    rslab = sl;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        rv[k] = ri[k] < p.ra.nr ? __ldg(p.ra.ring + (size_t)sl * p.ra.nr + ri[k]) : 0.f;
+                }
+            }
+        }
+        const bool zint = zo >= R && zo + R <= nz - 1;        // the window's planes all inside
+        const float rz = zint ? rz_in : recip_count(zo, nz, R);
+        const float nzf = zint ? (float)(2 * R + 1) : (float)(min(zo + R, nz - 1) - max(zo - R, 0) + 1);
+        const size_t ub = ((size_t)zo * ny + y0) * p.po + x0;  // the tile's first output of the plane
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k >= rows) continue;
+            const float2 sm = win[k];
+            const float s1 = sm.x, s2 = sm.y;
+            if (KIND == ZB_NOISE) {
+                // (explicit multiply-adds: every instance of this code rounds alike)
+                const float nin = nzf * nxy[k];                // in-bounds window size
+                // raw sums: S1 = S1' + nin*c, S2 = S2' + 2c*S1' + nin*c^2
+                const float nc = __fmul_rn(nin, c), m = __fmul_rn(s1 + nc, p.inv_wc);
+                float v;
+                if (nin == wcf) {                              // interior: shifted, cancellation-free
+                    const float e1 = __fmul_rn(s1, p.inv_wc);
+                    v = __fmaf_rn(s2, p.inv_wc, -__fmul_rn(e1, e1));
                 } else {
-                    const float2 mab = mul2(sm, rz);
-                    if (p.out_mode == 0) {
-                        const float g = gstage ? sguide[slot * G::GUIDE + (4 * rg + k) * TX + xc] : gv[k];
-                        float w = mab.x * g + mab.y;
-                        if (rings && w > 0.f && ri[k] < p.ra.nr) {     // masked voxels untouched
-                            const float w2 = w - p.ra.sc * rv[k];
-                            w = w2 > 0.f ? w2 : 0.f;
-                        }
-                        p.o0[o] = w;
-                    } else {
-                        p.o0[o] = mab.x; p.o1[o] = mab.y;
+                    const float S2 = __fmaf_rn(nc, c, __fmaf_rn(2.0f * c, s1, s2));
+                    v = __fmaf_rn(S2, p.inv_wc, -__fmul_rn(m, m));
+                }
+                if (v < 0.f) v = 0.f;
+                (p.o0 + ub)[off[k]] = m;
+                (p.o1 + ub)[off[k]] = v;
+                if (p.o2) {
+                    const size_t um = ((size_t)zo * ny + y0) * p.pmv + x0;
+                    const Off om = (Off)(4 * rg + k) * (Off)p.pmv + (Off)xc;
+                    (reinterpret_cast<float2*>(p.o2) + um)[om] = guided_mv(sm, ryk[k] * rz, c);
+                }
+            } else if (KIND == ZB_GUIDED_AB) {
+                (reinterpret_cast<float2*>(p.o0) + ub)[off[k]] = guided_ab(guided_mv(sm, ryk[k] * rz, c), eps);
+            } else {
+                const float2 mab = mul2(sm, rz);
+                if (p.out_mode == 0) {
+                    const float g = gstage ? sguide[slot * G::GUIDE + (4 * rg + k) * TX + xc] : gv[k];
+                    float w = __fmaf_rn(mab.x, g, mab.y);
+                    if (rings && w > 0.f && ri[k] < p.ra.nr) {     // masked voxels untouched
+                        const float w2 = __fmaf_rn(-p.ra.sc, rv[k], w);
+                        w = w2 > 0.f ? w2 : 0.f;
                     }
+                    (p.o0 + ub)[off[k]] = w;
+                } else {
+                    (p.o0 + ub)[off[k]] = mab.x;
+                    (p.o1 + ub)[off[k]] = mab.y;
                 }
             }
         }
@@ -593,7 +616,7 @@ inline dim3 grid_for(int kind, int nz, int ny, int nx, int r, int sms, int& zchu
 // outside. The encoder comes from the
 // driver through the runtime, so the library needs no link-time driver dependency. Returns
 // false when unavailable.
-inline bool make_tma_map(CUtensorMap* m, const float* base, int nz, int ny, int nx, int c, int bx, int by) {
+inline bool make_tma_map(CUtensorMap* m, const float* base, int nz, int ny, int nx, int pitch, int c, int bx, int by) {
     using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -608,14 +631,20 @@ inline bool make_tma_map(CUtensorMap* m, const float* base, int nz, int ny, int 
         else
             cudaGetLastError();
     });
-    if (!fn || ((uintptr_t)base & 15) || (nx % 4)) return false;
+    if (!fn || ((uintptr_t)base & 15) || pitch < nx || pitch % 4 || nx >= (1 << 24)) return false;
     const cuuint64_t dims[3] = {(cuuint64_t)nx * c, (cuuint64_t)ny, (cuuint64_t)nz};
-    const cuuint64_t strides[2] = {(cuuint64_t)nx * c * 4, (cuuint64_t)nx * ny * c * 4};
+    const cuuint64_t strides[2] = {(cuuint64_t)pitch * c * 4, (cuuint64_t)pitch * ny * c * 4};
     const cuuint32_t box[3] = {(cuuint32_t)(bx * c), (cuuint32_t)by, 1};
     const cuuint32_t es[3] = {1, 1, 1};
     return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, es,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Row pitches left at 0 are nx.
+inline void set_pitches(Params& p) {
+    for (int* q : {&p.pf0, &p.pg, &p.po, &p.pmv})
+        if (*q == 0) *q = p.nx;
 }
 
 template <int KIND, int R, bool VEC>
@@ -624,16 +653,21 @@ inline cudaError_t launch_r(const Params& p, dim3 grid, cudaStream_t st) {
     const size_t smem = Geo<R, C>::bytes;
     TmaMaps tm;
     memset(&tm, 0, sizeof tm);
-    const bool tma = VEC && make_tma_map(&tm.m0, p.f0, p.nz, p.ny, p.nx, C, SXW, Geo<R, C>::SY);
+    const bool tma = VEC && make_tma_map(&tm.m0, p.f0, p.nz, p.ny, p.nx, p.pf0, C, SXW, Geo<R, C>::SY);
     if (tma && out_kind(KIND) && p.out_mode == 0 && p.guide)
-        tm.guide = make_tma_map(&tm.m1, p.guide, p.nz, p.ny, p.nx, 1, TX, TY) ? 1 : 0;
+        tm.guide = make_tma_map(&tm.m1, p.guide, p.nz, p.ny, p.nx, p.pg, 1, TX, TY) ? 1 : 0;
     cudaError_t e;
     if (tma) {
         auto k = k_zbox<R, KIND, true, true>;
         if ((e = fy_smem_optin(k, smem)) != cudaSuccess) return e;
         return fy_launch_pdl(k, grid, dim3(NT), smem, st, p, tm);
     }
-    auto k = k_zbox<R, KIND, VEC, false>;
+    if (VEC && p.nx % 4 == 0) {                      // (16-byte copies must not straddle the rows' ends)
+        auto k = k_zbox<R, KIND, true, false>;
+        if ((e = fy_smem_optin(k, smem)) != cudaSuccess) return e;
+        return fy_launch_pdl(k, grid, dim3(NT), smem, st, p, tm);
+    }
+    auto k = k_zbox<R, KIND, false, false>;
     if ((e = fy_smem_optin(k, smem)) != cudaSuccess) return e;
     return fy_launch_pdl(k, grid, dim3(NT), smem, st, p, tm);
 }
@@ -643,15 +677,15 @@ inline cudaError_t launch_r(const Params& p, dim3 grid, cudaStream_t st) {
 // returns its number of work items, or -1 when the volume cannot use TMA staging (rows not
 // 16-byte aligned) or the encoder is unavailable.
 template <int KIND, int R>
-inline long long make_job_r(BoxJob& j, const Params& p, int sms, long long first) {
+inline long long make_job_r(BoxJob& j, Params p, int sms, long long first) {
     constexpr int C = out_kind(KIND) ? 2 : 1;
     memset(&j, 0, sizeof j);
+    set_pitches(p);
     j.p = p;
     const dim3 grid = grid_for(KIND, p.nz, p.ny, p.nx, R, sms, j.p.zchunk);
-    if (p.nx % 4 || ((uintptr_t)p.f0 & 15)) return -1;
-    if (!make_tma_map(&j.m0, p.f0, p.nz, p.ny, p.nx, C, SXW, Geo<R, C>::SY)) return -1;
+    if (!make_tma_map(&j.m0, p.f0, p.nz, p.ny, p.nx, p.pf0, C, SXW, Geo<R, C>::SY)) return -1;
     if (out_kind(KIND) && p.out_mode == 0 && p.guide)
-        j.guide = make_tma_map(&j.m1, p.guide, p.nz, p.ny, p.nx, 1, TX, TY) ? 1 : 0;
+        j.guide = make_tma_map(&j.m1, p.guide, p.nz, p.ny, p.nx, p.pg, 1, TX, TY) ? 1 : 0;
     j.tx = (int)grid.x;
     j.ty = (int)grid.y;
     j.first = first;
@@ -714,7 +748,8 @@ template <int KIND>
 inline cudaError_t launch(Params p, int r, int sms, cudaStream_t st) {
     const dim3 grid = grid_for(KIND, p.nz, p.ny, p.nx, r, sms, p.zchunk);
     auto al = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
-    const bool vec = p.nx % 4 == 0 && al(p.f0);
+    set_pitches(p);
+    const bool vec = p.pf0 % 4 == 0 && al(p.f0);
     switch (r * 2 + (vec ? 1 : 0)) {
         case 2: return launch_r<KIND, 1, false>(p, grid, st);
         case 3: return launch_r<KIND, 1, true>(p, grid, st);

@@ -302,7 +302,7 @@ void deconv_defaults(const fy_physics* p, int kind, double& param, double& fz2s)
 }
 
 // Enqueue the full deconvolution on st. src is device memory (u8 or f32), dst device f32.
-int enqueue_deconv(const void* src, int src_u8, double fmin, double fmax, float* dst, int nz, int ny,
+int enqueue_deconv(const void* src, int src_u8, double fmin, double fmax, float* dst, int dpitch, int nz, int ny,
                    int nx, const fy_physics* p, double param, int kind, double fz2s, cudaStream_t st,
                    const char* what) {
     fy::ThreadCtx& c = ctx();
@@ -317,7 +317,7 @@ int enqueue_deconv(const void* src, int src_u8, double fmin, double fmax, float*
     if (e != cudaSuccess) return fail_cuda(e, what);
     d.spec = c.spec.as<float2>();
     if ((rc = deconv_tables(d.g, p, param, kind, fz2s, st, d))) return rc;
-    d.src = src; d.src_u8 = src_u8; d.dst = dst;
+    d.src = src; d.src_u8 = src_u8; d.dst = dst; d.dpitch = dpitch;
     dewindow_params(fmin, fmax, d.lo, d.scale);
     if ((e = fy_launch_deconv(d, st)) != cudaSuccess) return fail_cuda(e, what);
     fy::count_launch(5);
@@ -340,7 +340,7 @@ int host_deconv(const float* in, float* out, int nz, int ny, int nx, const fy_ph
     if ((e = cudaMemcpyAsync(c.vin.p, in, n * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return fail_cuda(e, what);
     // dst aliases the device copy of src: P1 consumes src before P5 writes dst
-    if ((rc = enqueue_deconv(c.vin.p, 0, 0.0, 0.0, c.vin.as<float>(), nz, ny, nx, p, param, kind, fz2s, st,
+    if ((rc = enqueue_deconv(c.vin.p, 0, 0.0, 0.0, c.vin.as<float>(), nx, nz, ny, nx, p, param, kind, fz2s, st,
                              what)))
         return rc;
     if ((e = cudaMemcpyAsync(out, c.vin.p, n * sizeof(float), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
@@ -401,12 +401,17 @@ extern "C" int fy_gpu_deconvolve_ex(const void* d_in, int src_u8, double f32_min
                                     double param, int kind, double fz2_scale, void* stream) {
     fy::enter();
     if (!d_in || !d_out || !p) return fail(FY_EINVAL, "fy_gpu_deconvolve_ex: null pointer");
+    return fy_deconvolve_pitched(d_in, src_u8, f32_min, f32_max, d_out, nx, nz, ny, nx, p, param, kind, fz2_scale,
+                                 (cudaStream_t)stream);
+}
+
+int fy_deconvolve_pitched(const void* d_in, int src_u8, double f32_min, double f32_max, float* d_out, int dpitch, int nz,
+                          int ny, int nx, const fy_physics* p, double param, int kind, double fz2_scale, cudaStream_t st) {
     if (kind < 0 || kind > 2) return fail(FY_EINVAL, "fy_gpu_deconvolve_ex: kind %d", kind);
     int rc = fy::ensure_ctx();
     if (rc) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
     fy::ws_acquire(st);
-    rc = enqueue_deconv(d_in, src_u8 ? 1 : 0, f32_min, f32_max, d_out, nz, ny, nx, p, param, kind,
+    rc = enqueue_deconv(d_in, src_u8 ? 1 : 0, f32_min, f32_max, d_out, dpitch, nz, ny, nx, p, param, kind,
                         fz2_scale, st, "fy_gpu_deconvolve_ex");
     fy::ws_release(st);
     return rc;

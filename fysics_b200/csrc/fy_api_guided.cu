@@ -21,7 +21,7 @@ size_t guided_scratch_floats(int nz, int ny, int nx, int radius, int s) {
             return 3 * (size_t)lz * ly * lx + 4 * (size_t)lz * ly * lx;
         }
     }
-    return radius <= 4 ? fy_guided_fused_scratch_floats(n) : 4 * n;   // exact: a, b fields; generic: 4n
+    return radius <= 4 ? fy_guided_fused_scratch_floats(nz, ny, nx) : 4 * n;   // exact: a, b fields; generic: 4n
 }
 
 int enqueue_guided(const float* in, float* out, float* scratch, int nz, int ny, int nx, int radius,

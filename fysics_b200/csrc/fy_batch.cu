@@ -100,7 +100,7 @@ extern "C" int fy_gpu_restore_u8_batch(const fy_batch_cube* cubes, int n, const 
         const size_t vox = (size_t)q.nz * q.ny * q.nx;
         off_dec[i] = arena; arena += al256(vox * sizeof(float));
         off_scr[i] = arena; arena += al256(fy_noise_scratch_floats(vox) * sizeof(float));
-        off_mv[i] = arena; arena += al256(fy_guided_fused_scratch_floats(vox) * sizeof(float));
+        off_mv[i] = arena; arena += al256(fy_guided_fused_scratch_floats(q.nz, q.ny, q.nx) * sizeof(float));
         off_ctl[i] = arena; arena += al256(fy_noise_ctl_bytes());
         params[i] = cfg->deconv_param;
         fz2ss[i] = cfg->fz2_scale;
@@ -177,6 +177,7 @@ extern "C" int fy_gpu_restore_u8_batch(const fy_batch_cube* cubes, int n, const 
         d.src = q.u8;
         d.src_u8 = 1;
         d.dst = reinterpret_cast<float*>(A + off_dec[i]);
+        d.dpitch = q.nx;
         d.spec = c.bspec[i % K].as<float2>();
         float* mv = reinterpret_cast<float*>(A + off_mv[i]);
         const fyzb::Params ps = fy_noise_stats_params(d.dst, q.nz, q.ny, q.nx, win, scr[i], mv);

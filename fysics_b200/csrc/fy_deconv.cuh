@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_y_inv(float2* __restrict__ spe
 // ---------------------------------------------------------------- P5
 // Line-major like P1; the two output rows of a line are written VEC floats at a time.
 template <int N, int E, int VEC>
-__global__ void __launch_bounds__(KB<E>::nt, 2) k_x_inv(const float2* __restrict__ spec, float* __restrict__ dst,
+__global__ void __launch_bounds__(KB<E>::nt, 2) k_x_inv(const float2* __restrict__ spec, float* __restrict__ dst, int dpitch,
                                                         SpecGeom g, const __grid_constant__ FftPlan pl,
                                                         const float2* __restrict__ tw, float invN, int wlog,
                                                         FastDiv dchunk, FastDiv dhx) {
@@ -383,14 +383,14 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_x_inv(const float2* __restrict
         if (qa >= Q) continue;
         const float2* v = s + l * LPX + x;
         if (VEC == 4) {
-            *reinterpret_cast<float4*>(dst + qa * g.nx + x) =
+            *reinterpret_cast<float4*>(dst + qa * dpitch + x) =
                 make_float4(v[0].x * invN, v[1].x * invN, v[2].x * invN, v[3].x * invN);
             if (qb < Q)
-                *reinterpret_cast<float4*>(dst + qb * g.nx + x) =
+                *reinterpret_cast<float4*>(dst + qb * dpitch + x) =
                     make_float4(v[0].y * invN, v[1].y * invN, v[2].y * invN, v[3].y * invN);
         } else {
-            dst[qa * g.nx + x] = v[0].x * invN;
-            if (qb < Q) dst[qb * g.nx + x] = v[0].y * invN;
+            dst[qa * dpitch + x] = v[0].x * invN;
+            if (qb < Q) dst[qb * dpitch + x] = v[0].y * invN;
         }
     }
 }
@@ -478,7 +478,7 @@ cudaError_t fy_deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
         const size_t smem = (size_t)t.W * (g.px + 1) * sizeof(float2) + (size_t)g.px * sizeof(float2);
         const unsigned grid = (unsigned)((Q + 2 * t.W - 1) / (2 * t.W));
         const float invN = 1.0f / ((float)g.pz * (float)g.py * (float)g.px);   // paganin.c:263
-        const bool vec = g.nx % 4 == 0 && ((uintptr_t)d.dst % 16) == 0;
+        const bool vec = g.nx % 4 == 0 && d.dpitch % 4 == 0 && ((uintptr_t)d.dst % 16) == 0;
         return with_e(g.px, [&](auto ec) -> cudaError_t {
             constexpr int E = decltype(ec)::value;
             cudaError_t e2 = cudaSuccess;
@@ -486,13 +486,13 @@ cudaError_t fy_deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
             if (vec) {
                 auto k = k_x_inv<N, E, 4>;
                 if ((e2 = fy_smem_optin(k, smem)) != cudaSuccess) return e2;
-                if ((e2 = fy_launch_pdl(k, dim3(grid), dim3(t.NT), smem, st, (const float2*)d.spec, d.dst, g, d.plx,
+                if ((e2 = fy_launch_pdl(k, dim3(grid), dim3(t.NT), smem, st, (const float2*)d.spec, d.dst, d.dpitch, g, d.plx,
                                         d.twx, invN, t.wlog, dch, dhx)) != cudaSuccess)
                     return e2;
             } else {
                 auto k = k_x_inv<N, E, 1>;
                 if ((e2 = fy_smem_optin(k, smem)) != cudaSuccess) return e2;
-                if ((e2 = fy_launch_pdl(k, dim3(grid), dim3(t.NT), smem, st, (const float2*)d.spec, d.dst, g, d.plx,
+                if ((e2 = fy_launch_pdl(k, dim3(grid), dim3(t.NT), smem, st, (const float2*)d.spec, d.dst, d.dpitch, g, d.plx,
                                         d.twx, invN, t.wlog, dch, dhx)) != cudaSuccess)
                     return e2;
             }

@@ -94,23 +94,26 @@ cudaError_t box3(const float* in, float* out, float* tmp, int nz, int ny, int nx
 int fy_guided_fused_max_radius() { return 4; }
 
 static size_t round64(size_t v) { return (v + 63) & ~(size_t)63; }
-size_t fy_guided_fused_scratch_floats(size_t n) { return 2 * round64(n); }
+size_t fy_guided_fused_scratch_floats(int nz, int ny, int nx) { return 2 * round64((size_t)nz * ny * fy_pitch(nx)); }
 
 // Exact guided filter for r in [1, 4] as two z-sliding box passes (fy_zbox.cuh):
 // in -> interleaved (a, b) pairs into ab_ws, then box(a), box(b) -> out. ab_ws holds
 // fy_guided_fused_scratch_floats(n) floats; out may alias in. mode 1 writes box(a) to out
-// and box(b) to out_b instead of the filtered volume.
+// and box(b) to out_b instead of the filtered volume. The pairs' rows are fy_pitch(nx) voxels apart, so
+// the second pass stages them by TMA whatever nx is.
 cudaError_t fy_launch_guided_fused(const float* in, float* out, float* out_b, float* ab_ws, int nz, int ny, int nx,
                                    int r, float eps, int mode, int sms, cudaStream_t st, const float* eps_ptr,
-                                   const RingApply* rings) {
+                                   const RingApply* rings, int in_pitch) {
     if (r < 1 || r > 4) return cudaErrorInvalidValue;
     fyzb::Params p{};
     p.nz = nz; p.ny = ny; p.nx = nx;
+    p.pf0 = in_pitch; p.po = fy_pitch(nx);
     p.f0 = in; p.o0 = ab_ws; p.eps = eps; p.eps_ptr = eps_ptr;
     cudaError_t e = fyzb::launch<fyzb::ZB_GUIDED_AB>(p, r, sms, st);
     if (e != cudaSuccess) return e;
     fyzb::Params q{};
     q.nz = nz; q.ny = ny; q.nx = nx;
+    q.pf0 = fy_pitch(nx); q.pg = in_pitch;
     q.f0 = ab_ws; q.guide = in; q.o0 = out; q.o1 = out_b; q.out_mode = mode;
     if (rings && mode == 0) q.ra = *rings;
     return fyzb::launch<fyzb::ZB_GUIDED_OUT>(q, r, sms, st);
@@ -122,10 +125,11 @@ cudaError_t fy_launch_guided_fused(const float* in, float* out, float* out_b, fl
 // *eps_ptr) must be > 0.
 cudaError_t fy_launch_guided_apply_mv(const float* mv, const float* in, float* out, int nz, int ny, int nx, int r,
                                       float eps, int sms, cudaStream_t st, const float* eps_ptr,
-                                      const RingApply* rings) {
+                                      const RingApply* rings, int in_pitch) {
     if (r < 1 || r > 4) return cudaErrorInvalidValue;
     fyzb::Params q{};
     q.nz = nz; q.ny = ny; q.nx = nx;
+    q.pf0 = fy_pitch(nx); q.pg = in_pitch;
     q.f0 = mv; q.guide = in; q.o0 = out; q.out_mode = 0; q.eps = eps; q.eps_ptr = eps_ptr;
     if (rings) q.ra = *rings;
     return fyzb::launch<fyzb::ZB_GUIDED_OUT_MV>(q, r, sms, st);
@@ -133,15 +137,15 @@ cudaError_t fy_launch_guided_apply_mv(const float* mv, const float* in, float* o
 
 // ---------------------------------------------------------------- fast (s-decimated) variant
 namespace {
-// Il[z][y][x] = in[(z*s)][(y*s)][(x*s)]  (guided.c:163-168: decimation, not a mean)
+// Il[z][y][x] = in[(z*s)][(y*s)][(x*s)]  (guided.c:163-168: decimation, not a mean); rows of Il lp apart
 __global__ void k_decimate(const float* __restrict__ in, float* __restrict__ lo, int ny, int nx,
-                           int lz, int ly, int lx, int s) {
+                           int lz, int ly, int lx, int lp, int s) {
     const size_t nl = (size_t)lz * ly * lx;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += (size_t)gridDim.x * blockDim.x) {
         const int x = (int)(i % lx);
         const size_t zy = i / lx;
         const int y = (int)(zy % ly), z = (int)(zy / ly);
-        lo[i] = __ldg(in + ((size_t)z * s * ny + (size_t)y * s) * nx + (size_t)x * s);
+        lo[zy * lp + x] = __ldg(in + ((size_t)z * s * ny + (size_t)y * s) * nx + (size_t)x * s);
     }
 }
 
@@ -185,7 +189,7 @@ __global__ void __launch_bounds__(256) k_upsample_apply(const float* __restrict_
 
 size_t fy_guided_fast_scratch_floats(int lz, int ly, int lx) {
     const size_t nl = round64((size_t)lz * ly * lx);
-    return 3 * nl + fy_guided_fused_scratch_floats((size_t)lz * ly * lx);
+    return 2 * nl + round64((size_t)lz * ly * fy_pitch(lx)) + fy_guided_fused_scratch_floats(lz, ly, lx);
 }
 
 // Fast guided filter (s >= 2, all low dims >= 2, rl = max(1, r/s) <= 4).
@@ -194,11 +198,11 @@ cudaError_t fy_launch_guided_fast(const float* in, float* out, float* ws, int nz
                                   float eps, int s, int sms, cudaStream_t st, int& launches, const float* eps_ptr) {
     const int lz = (nz + s - 1) / s, ly = (ny + s - 1) / s, lx = (nx + s - 1) / s;
     const size_t nl = (size_t)lz * ly * lx, nlr = round64(nl);
-    float *il = ws, *ma = ws + nlr, *mb = ws + 2 * nlr, *ab = ws + 3 * nlr;
+    float *ma = ws, *mb = ws + nlr, *il = ws + 2 * nlr, *ab = il + round64((size_t)lz * ly * fy_pitch(lx));
     int rl = r / s;
     if (rl < 1) rl = 1;
-    k_decimate<<<grid_1d(nl), 256, 0, st>>>(in, il, ny, nx, lz, ly, lx, s);
-    cudaError_t e = fy_launch_guided_fused(il, ma, mb, ab, lz, ly, lx, rl, eps, 1, sms, st, eps_ptr);
+    k_decimate<<<grid_1d(nl), 256, 0, st>>>(in, il, ny, nx, lz, ly, lx, fy_pitch(lx), s);
+    cudaError_t e = fy_launch_guided_fused(il, ma, mb, ab, lz, ly, lx, rl, eps, 1, sms, st, eps_ptr, nullptr, fy_pitch(lx));
     if (e != cudaSuccess) return e;
     const int tpb = nx < 256 ? (nx + 31) / 32 * 32 : 256;     // whole warps across a row
     dim3 grid(ceil_div_i(nx, tpb), ny, nz);

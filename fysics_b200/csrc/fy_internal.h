@@ -14,7 +14,8 @@ struct DeconvLaunch {
     const void* src;          // f32 or u8 volume (nz,ny,nx)
     int src_u8;               // 1: u8 source dewindowed as lo + u8*scale (stream.c:41-46)
     float lo, scale;
-    float* dst;               // f32 (nz,ny,nx); may alias src when src is f32
+    float* dst;               // f32 (nz,ny,nx), rows dpitch floats apart; may alias src when src is f32 (dpitch nx)
+    int dpitch;
     float2* spec;             // nz * py * hxp complex workspace
     SpecGeom g;
     FftPlan plx, ply, plz;
@@ -36,6 +37,9 @@ size_t fy_deconv_table_bytes(const SpecGeom& g);
 double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double param, int kind, double fz2s, void* host);
 int fy_deconv_setup(int nz, int ny, int nx, const fy_physics* p, double& param, int kind, double& fz2s,
                     double fmin, double fmax, DeconvLaunch& d, const char* what);
+// fy_gpu_deconvolve_ex with output rows dpitch floats apart.
+int fy_deconvolve_pitched(const void* d_in, int src_u8, double f32_min, double f32_max, float* d_out, int dpitch, int nz,
+                          int ny, int nx, const fy_physics* p, double param, int kind, double fz2_scale, cudaStream_t st);
 cudaError_t fy_launch_cfft3d(float2* c, int nz, int ny, int nx, int nxp, int sign, cudaStream_t st);
 
 // Elementwise stream ops (stream.c)
@@ -60,12 +64,16 @@ struct RingApply {
 // Fill `ra` from a device ring handle (fy_api_dering.cu).
 void fy_dering_ring_args(const fy_gpu_dering* h, long z0, long y0, long x0, double scale, RingApply* ra);
 
-// exact r <= 4: ab_ws holds fy_guided_fused_scratch_floats(n); out may alias in
-size_t fy_guided_fused_scratch_floats(size_t n);
+// Row pitch (voxels) of a field of the library's own: rows begin 16-byte aligned, as the box passes'
+// TMA staging needs.
+inline int fy_pitch(int nx) { return (nx + 3) & ~3; }
+// exact r <= 4: ab_ws holds fy_guided_fused_scratch_floats(); out may alias in. in_pitch: floats per row
+// of `in` (0: nx)
+size_t fy_guided_fused_scratch_floats(int nz, int ny, int nx);
 size_t fy_guided_fast_scratch_floats(int lz, int ly, int lx);
 cudaError_t fy_launch_guided_fused(const float* in, float* out, float* out_b, float* ab_ws, int nz, int ny, int nx,
                                    int r, float eps, int mode, int sms, cudaStream_t st,
-                                   const float* eps_ptr = nullptr, const RingApply* rings = nullptr);
+                                   const float* eps_ptr = nullptr, const RingApply* rings = nullptr, int in_pitch = 0);
 cudaError_t fy_launch_guided_generic(const float* in, float* out, float* ws, int nz, int ny, int nx, int r,
                                      float eps, cudaStream_t st, int& launches);
 cudaError_t fy_launch_guided_fast(const float* in, float* out, float* ws, int nz, int ny, int nx, int r,
@@ -76,14 +84,14 @@ cudaError_t fy_launch_box_mean(const float* in, float* out, float* tmp, int nz, 
 // output pass from guided (mean, var) pairs written by the noise statistics pass (r = win/2)
 cudaError_t fy_launch_guided_apply_mv(const float* mv, const float* in, float* out, int nz, int ny, int nx, int r,
                                       float eps, int sms, cudaStream_t st, const float* eps_ptr,
-                                      const RingApply* rings);
+                                      const RingApply* rings, int in_pitch = 0);
 
 // Noise model (fy_noise.cu)
 size_t fy_noise_ctl_bytes();
 size_t fy_noise_scratch_floats(size_t n);
 cudaError_t fy_launch_estimate_noise(const float* in, int nz, int ny, int nx, int win, double flat_pct,
                                      double ref_intensity, float* scratch, void* ctl_mem, int sms,
-                                     cudaStream_t st, int& launches, float* guided_mv = nullptr);
+                                     cudaStream_t st, int& launches, float* guided_mv = nullptr, int in_pitch = 0);
 cudaError_t fy_noise_read(const void* ctl_mem, double* g, double* b, double* noise_ref, double* ref_intensity,
                           int* used, cudaStream_t st);
 const float* fy_noise_eps_ptr(const void* ctl_mem);

@@ -1388,7 +1388,7 @@ struct NoiseLaunch {
 // (a batch runs it for all volumes at once before the sequence).
 cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int nx, int win, double flat_pct,
                            double ref_intensity, float* scratch, void* ctl_mem, int sms, int& launches,
-                           float* guided_mv, bool stats) {
+                           float* guided_mv, bool stats, int in_pitch = 0) {
     cudaStream_t st = L.st;
     NoiseCtl* ctl = (NoiseCtl*)ctl_mem;
     const long long n = (long long)nz * ny * nx;
@@ -1419,6 +1419,7 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
         sp.nz = nz; sp.ny = ny; sp.nx = nx;
         sp.f0 = in; sp.o0 = mean; sp.o1 = var; sp.o2 = guided_mv;
         sp.inv_wc = inv_wc; sp.wci = win * win * win;
+        sp.pf0 = in_pitch; sp.pmv = fy_pitch(nx);
         cudaError_t e0 = fyzb::launch<fyzb::ZB_NOISE>(sp, r, sms, st);
         if (e0 != cudaSuccess) return e0;
         ++launches;
@@ -1458,16 +1459,16 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
 
 // Enqueue the whole estimate. scratch: fy_noise_scratch_floats(n) floats; ctl:
 // fy_noise_ctl_bytes(). Supports win in {3..9} (r = win/2 <= 4). guided_mv (optional,
-// 2n floats): the statistics pass also writes the guided filter's (mean, var) pairs of the
-// same window, for fy_launch_guided_apply_mv with r = win/2.
+// fy_guided_fused_scratch_floats, rows fy_pitch(nx) voxels apart): the statistics pass also writes the guided filter's (mean, var) pairs of the
+// same window, for fy_launch_guided_apply_mv with r = win/2. in_pitch: floats per row of `in` (0: nx).
 // Every kernel runs as a programmatic dependent launch; the first failed launch is returned.
 cudaError_t fy_launch_estimate_noise(const float* in, int nz, int ny, int nx, int win, double flat_pct,
                                      double ref_intensity, float* scratch, void* ctl_mem, int sms,
-                                     cudaStream_t st, int& launches, float* guided_mv) {
+                                     cudaStream_t st, int& launches, float* guided_mv, int in_pitch) {
     NoiseLaunch L;
     L.st = st;
     cudaError_t e = noise_sequence(L, in, nz, ny, nx, win, flat_pct, ref_intensity, scratch, ctl_mem, sms, launches,
-                                   guided_mv, true);
+                                   guided_mv, true, in_pitch);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

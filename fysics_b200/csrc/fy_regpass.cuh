@@ -267,7 +267,7 @@ k_row_fwd(const T* __restrict__ src, float lo, float scale, float2* __restrict__
 // transform, crop, 1/N.
 template <int N, bool CROP>
 __global__ void __launch_bounds__(Row<N>::NT, Row<N>::minb)
-k_row_inv(const float2* __restrict__ spec, float* __restrict__ dst, SpecGeom g, const float2* __restrict__ tw, float invN) {
+k_row_inv(const float2* __restrict__ spec, float* __restrict__ dst, int dpitch, SpecGeom g, const float2* __restrict__ tw, float invN) {
     fy_pdl_wait();
     extern __shared__ float4 smem4[];
     constexpr int E = elems(N), TPL = tpl(N), H = E / 2;
@@ -310,8 +310,8 @@ k_row_inv(const float2* __restrict__ spec, float* __restrict__ dst, SpecGeom g, 
     load_tail_twiddles<N>(stw, tw);
     __syncthreads();
     row_fft<N, +1>(v, ln.s, t, stw);
-    float* da = dst + ln.qa * g.nx;
-    float* db = da + g.nx;
+    float* da = dst + ln.qa * dpitch;
+    float* db = da + dpitch;
 #pragma unroll
     for (int m = 0; m < E; ++m) {
         const int x = t + TPL * m;
@@ -377,8 +377,8 @@ cudaError_t deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
         const int nt = row_threads<N>(5);
         const size_t smem = Row<N>::tw_smem + Row<N>::warp_smem * (nt / 32);
         const float invN = 1.0f / ((float)g.pz * (float)g.py * (float)g.px);   // paganin.c:263
-        if (g.nx != N) return launch(k_row_inv<N, true>, rows(nt), nt, smem, st, (const float2*)d.spec, d.dst, g, d.twx, invN);
-        return launch(k_row_inv<N, false>, rows(nt), nt, smem, st, (const float2*)d.spec, d.dst, g, d.twx, invN);
+        if (g.nx != N) return launch(k_row_inv<N, true>, rows(nt), nt, smem, st, (const float2*)d.spec, d.dst, d.dpitch, g, d.twx, invN);
+        return launch(k_row_inv<N, false>, rows(nt), nt, smem, st, (const float2*)d.spec, d.dst, d.dpitch, g, d.twx, invN);
     }
     default: return cudaErrorInvalidValue;
     }

@@ -16,9 +16,6 @@ extern "C" int fy_gpu_dering_finalize(fy_gpu_dering* h, int hp_win, unsigned int
                                       double max_amp, void* stream);
 extern "C" int fy_gpu_dering_apply(const fy_gpu_dering* h, float* d_f, long z0, long y0, long x0, long dz, long dy,
                                    long dx, double scale, void* stream);
-extern "C" int fy_gpu_deconvolve_ex(const void* d_in, int src_u8, double f32_min, double f32_max, float* d_out,
-                                    int nz, int ny, int nx, const fy_physics* p, double param, int kind,
-                                    double fz2_scale, void* stream);
 
 extern "C" void fy_restore_cfg_default(fy_restore_cfg* c) {
     c->deconv_kind = 0;
@@ -79,12 +76,15 @@ extern "C" int fy_gpu_restore_u8(const unsigned char* d_u8, float* d_out, int nz
     }
     fy::ws_acquire(st);
     cudaError_t e;
-    if ((e = c.aux2.ensure(n * sizeof(float))) != cudaSuccess) return fail_cuda(e, what);
+    // the box passes take rows of any length through TMA when they begin 16-byte aligned: rows of the
+    // deconvolved volume are padded to 4 voxels (the decimated filter reads dense rows)
+    const int dp = cfg->guided_s > 1 ? nx : fy_pitch(nx);
+    if ((e = c.aux2.ensure((size_t)nz * ny * dp * sizeof(float))) != cudaSuccess) return fail_cuda(e, what);
     float* dec = c.aux2.as<float>();
-    fy::ws_release(st);      // deconvolve_ex re-acquires the shared workspaces
+    fy::ws_release(st);      // the deconvolution re-acquires the shared workspaces
     // 2. dewindow + deconvolution into `dec`
-    if ((rc = fy_gpu_deconvolve_ex(d_u8, 1, f32_min, f32_max, dec, nz, ny, nx, p, cfg->deconv_param,
-                                   cfg->deconv_kind, cfg->fz2_scale, stream)))
+    if ((rc = fy_deconvolve_pitched(d_u8, 1, f32_min, f32_max, dec, dp, nz, ny, nx, p, cfg->deconv_param,
+                                    cfg->deconv_kind, cfg->fz2_scale, st)))
         return rc;
     fy::ws_acquire(st);
     // 3. noise model on the deconvolved volume -> device eps. When the noise window is the
@@ -96,13 +96,13 @@ extern "C" int fy_gpu_restore_u8(const unsigned char* d_u8, float* d_out, int nz
     const bool shared_window = noise && cfg->guided_s <= 1 && win == 2 * radius + 1;
     const size_t mv_off = fy_noise_scratch_floats(n);
     if (noise) {
-        const size_t need = mv_off + (shared_window ? fy_guided_fused_scratch_floats(n) : 0);
+        const size_t need = mv_off + (shared_window ? fy_guided_fused_scratch_floats(nz, ny, nx) : 0);
         if ((e = c.aux.ensure(need * sizeof(float))) != cudaSuccess) return fail_cuda(e, what);
         if ((e = c.small.ensure(fy_noise_ctl_bytes())) != cudaSuccess) return fail_cuda(e, what);
         double pct = cfg->noise_flat_pct <= 0 ? 10.0 : cfg->noise_flat_pct;
         if ((e = fy_launch_estimate_noise(dec, nz, ny, nx, win, pct, cfg->noise_ref_intensity, c.aux.as<float>(),
                                           c.small.p, c.sms, st, launches,
-                                          shared_window ? c.aux.as<float>() + mv_off : nullptr)) != cudaSuccess)
+                                          shared_window ? c.aux.as<float>() + mv_off : nullptr, dp)) != cudaSuccess)
             return fail_cuda(e, what);
         eps_ptr = fy_noise_eps_ptr(c.small.p);
         fy_prof_mark(st, "noise");
@@ -131,7 +131,7 @@ extern "C" int fy_gpu_restore_u8(const unsigned char* d_u8, float* d_out, int nz
             e = fy_launch_guided_fast(dec, d_out, c.vout.as<float>(), nz, ny, nx, radius, eps, s, c.sms, st, launches,
                                       eps_ptr);
         } else {
-            if ((e = c.aux.ensure(fy_guided_fused_scratch_floats(n) * sizeof(float))) != cudaSuccess)
+            if ((e = c.aux.ensure(fy_guided_fused_scratch_floats(nz, ny, nx) * sizeof(float))) != cudaSuccess)
                 return fail_cuda(e, what);
             e = fy_launch_guided_fused(dec, d_out, nullptr, c.aux.as<float>(), nz, ny, nx, radius, eps, 0, c.sms, st,
                                        eps_ptr);
@@ -143,14 +143,14 @@ extern "C" int fy_gpu_restore_u8(const unsigned char* d_u8, float* d_out, int nz
         if (cfg->dering) fy_dering_ring_args(cfg->dering, cfg->z0, cfg->y0, cfg->x0, cfg->dering_scale, &ra);
         if (shared_window) {
             e = fy_launch_guided_apply_mv(c.aux.as<float>() + mv_off, dec, d_out, nz, ny, nx, radius, eps, c.sms, st,
-                                          eps_ptr, cfg->dering ? &ra : nullptr);
+                                          eps_ptr, cfg->dering ? &ra : nullptr, dp);
             launches += 1;
         } else {
             // a, b reuse the noise statistics' scratch: the model is final by now (stream order)
-            if ((e = c.aux.ensure(fy_guided_fused_scratch_floats(n) * sizeof(float))) != cudaSuccess)
+            if ((e = c.aux.ensure(fy_guided_fused_scratch_floats(nz, ny, nx) * sizeof(float))) != cudaSuccess)
                 return fail_cuda(e, what);
             e = fy_launch_guided_fused(dec, d_out, nullptr, c.aux.as<float>(), nz, ny, nx, radius, eps, 0, c.sms, st,
-                                       eps_ptr, cfg->dering ? &ra : nullptr);
+                                       eps_ptr, cfg->dering ? &ra : nullptr, dp);
             launches += 2;
         }
         rings_done = cfg->dering != nullptr;
@@ -178,9 +178,9 @@ int fy_restore_reserve(int nz, int ny, int nx) {
     if (rc) return rc;
     fy::ThreadCtx& c = ctx();
     const size_t n = (size_t)nz * ny * nx;
-    size_t aux = fy_noise_scratch_floats(n) + fy_guided_fused_scratch_floats(n);   // noise + guided (mean, var)
+    size_t aux = fy_noise_scratch_floats(n) + fy_guided_fused_scratch_floats(nz, ny, nx);   // noise + guided (mean, var)
     cudaError_t e;
-    if ((e = c.aux2.ensure(n * sizeof(float))) != cudaSuccess || (e = c.aux.ensure(aux * sizeof(float))) != cudaSuccess ||
+    if ((e = c.aux2.ensure((size_t)nz * ny * fy_pitch(nx) * sizeof(float))) != cudaSuccess || (e = c.aux.ensure(aux * sizeof(float))) != cudaSuccess ||
         (e = c.small.ensure(fy_noise_ctl_bytes() + 256)) != cudaSuccess)
         return fail_cuda(e, "fy_restore_reserve");
     return FY_OK;

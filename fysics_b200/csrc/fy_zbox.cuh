@@ -260,6 +260,34 @@ FY_D bool zbox_tile(const Params& p, const TmaRef& tm, int bx, int by, int bz, u
     auto guide_slot = [&](int slot, int zi) -> float* {
         return gstage && zi - R >= zs && zi - R < ze ? sguide + slot * G::GUIDE : nullptr;
     };
+    // 4-byte copies: the elements of a staged plane that this thread copies, every NT-th, as offsets in
+    // a plane of the volume (bit i of sok: element i lies inside it)
+    constexpr int SPT = C == 1 && !TMA && !VEC ? (G::SY * G::RW + NT - 1) / NT : 1;
+    size_t soff[SPT];
+    unsigned sok = 0;
+    if (SPT > 1) {
+#pragma unroll
+        for (int i = 0; i < SPT; ++i) {
+            const int k = t + i * NT, yy = k / G::RW, gy = y0 - R + yy, gxk = x0 - 4 + (k - yy * G::RW);
+            const bool in = k < G::SY * G::RW && gy >= 0 && gy < ny && gxk >= 0 && gxk < nx;
+            soff[i] = in ? (size_t)gy * p.pf0 + gxk : 0;
+            sok |= (unsigned)in << i;
+        }
+    }
+    auto stage_in = [&](int s, int zi) {                           // plane zi into slot s by asynchronous copies
+        float* dst = stage + s * G::STAGE;
+        if (SPT == 1) {
+            stage_plane<R, C, VEC>(dst, p, zi, x0, y0);
+            return;
+        }
+        const bool zin = zi >= 0 && zi < nz;
+        const float* src = p.f0 + (size_t)(zin ? zi : 0) * ny * p.pf0;
+        const unsigned okm = zin ? sok : 0u;
+#pragma unroll
+        for (int i = 0; i < SPT; ++i)
+            if ((i + 1) * NT <= G::SY * G::RW || t + i * NT < G::SY * G::RW)
+                cp4(dst + t + i * NT, src + soff[i], (okm >> i) & 1u);
+    };
     if (TMA) {
         if (t == 0) {
             for (int s = 0; s < NS; ++s) mbar_init(&bars[s], 1);
@@ -273,7 +301,7 @@ FY_D bool zbox_tile(const Params& p, const TmaRef& tm, int bx, int by, int bz, u
     } else {
 #pragma unroll
         for (int s = 0; s < NS - 1; ++s) {
-            if (zfirst + s < zend) stage_plane<R, C, VEC>(stage + s * G::STAGE, p, zfirst + s, x0, y0);
+            if (zfirst + s < zend) stage_in(s, zfirst + s);
             cp_commit();
         }
     }
@@ -356,7 +384,7 @@ FY_D bool zbox_tile(const Params& p, const TmaRef& tm, int bx, int by, int bz, u
             cp_wait<NS - 2>();
             __syncthreads();             // plane zi landed for every thread; xs free again
             const int zn = zi + NS - 1;
-            if (zn < zend) stage_plane<R, C, VEC>(stage + ((zn - zfirst) & (NS - 1)) * G::STAGE, p, zn, x0, y0);
+            if (zn < zend) stage_in((zn - zfirst) & (NS - 1), zn);
             cp_commit();
         }
         const int zo = zi - R;

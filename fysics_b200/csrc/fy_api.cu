@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "fy_context.h"
+#include "fy_hostcopy.h"
 
 using fy::ctx;
 using fy::fail;
@@ -337,17 +338,15 @@ int host_deconv(const float* in, float* out, int nz, int ny, int nx, const fy_ph
     fy::ws_acquire(st);
     cudaError_t e = c.vin.ensure(n * sizeof(float));
     if (e != cudaSuccess) return fail_cuda(e, what);
-    if ((e = cudaMemcpyAsync(c.vin.p, in, n * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess)
-        return fail_cuda(e, what);
+    fy::HostCopy copy(n * sizeof(float));
+    if ((e = copy.to_device(c.vin.p, in, n * sizeof(float), st)) != cudaSuccess) return fail_cuda(e, what);
     // dst aliases the device copy of src: P1 consumes src before P5 writes dst
     if ((rc = enqueue_deconv(c.vin.p, 0, 0.0, 0.0, c.vin.as<float>(), nx, nz, ny, nx, p, param, kind, fz2s, st,
                              what)))
         return rc;
-    if ((e = cudaMemcpyAsync(out, c.vin.p, n * sizeof(float), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-        return fail_cuda(e, what);
     fy::ws_release(st);
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, what);
-    return FY_OK;
+    e = copy.from_device(out, c.vin.p, n * sizeof(float), st);
+    return e == cudaSuccess ? FY_OK : fail_cuda(e, what);
 }
 }  // namespace
 

@@ -11,7 +11,7 @@
 //   air zero        k_box_line_smem x3 over the 2x-decimated orig (the sliding sums of
 //                   guided.c:34-98; the last pass also bins the means), k_air_cut (stream.c:138-168 and
 //                   pipeline.c:330-364), k_air_apply (the texture split, :355-399), which
-//                   also writes the despeckle's x-run labels
+//                   also writes the despeckle's material bits and x-run heads
 //   despeckle       union-find over 6-connected material (:223-250, :400-405): k_cc_union,
 //                   k_cc_count (roots, sizes, face contact); the zeroing of small interior
 //                   components is applied by the quantiser
@@ -432,27 +432,8 @@ __global__ void __launch_bounds__(256) k_air_cut(TileCtl* ctl, int air_cut_u8, i
     ctl->cutf_tex = __fmul_rn((float)ct, 1.0f / 255.0f);
 }
 
-// The x of the first voxel of this voxel's material run within the CTA's row segment
-// (threads = consecutive x, whole warps): the warp's own ballot, then the earlier warps'
-// ballots in shared memory. Every thread of the CTA must call it (two barriers).
-__device__ __forceinline__ int run_head(bool mat, unsigned* wbits) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned bits = __ballot_sync(0xffffffffu, mat);
-    if (lane == 0) wbits[warp] = bits;
-    __syncthreads();
-    int head = 0;
-    const unsigned gaps = ~bits & ((1u << lane) - 1u);
-    if (gaps) {
-        head = warp * 32 + 32 - __clz(gaps);
-    } else {
-        for (int w = warp - 1; w >= 0; --w) {
-            const unsigned g = ~wbits[w];
-            if (g) { head = w * 32 + 32 - __clz(g); break; }
-        }
-    }
-    __syncthreads();                         // wbits is rewritten by the next row
-    return head;
-}
+// Rows (x lines) taken by one CTA of the row kernels: a warp each, no barrier.
+constexpr int kRowWarps = 8;
 
 struct AirArgs {
     float* f;                 // may alias orig: each voxel reads orig and writes f at itself
@@ -461,63 +442,78 @@ struct AirArgs {
     const TileCtl* ctl;
     long nz, ny, nx, lz, ly, lx;
     int lowres;
-    int* lab;                 // despeckle on: x-run labels of the material (f > 0) written here
+    unsigned* mask;           // despeckle on: a bit per voxel, material (f > 0), rows of `words` words
+    int words;
+    int* lab;                 // despeckle on: parents of the run heads (k_cc_union's nodes)
     unsigned* info;
 };
 
-__device__ __forceinline__ float blend4(const float* s, size_t r00, size_t r01, size_t r10, size_t r11, long k,
-                                        float w00, float w01, float w10, float w11) {
-    return __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(w00, s[r00 + k]), __fmul_rn(w01, s[r01 + k])),
-                               __fmul_rn(w10, s[r10 + k])),
-                     __fmul_rn(w11, s[r11 + k]));
+__device__ __forceinline__ float blend4(float s00, float s01, float s10, float s11, float w00, float w01, float w10,
+                                        float w11) {
+    return __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(w00, s00), __fmul_rn(w01, s01)), __fmul_rn(w10, s10)),
+                     __fmul_rn(w11, s11));
 }
 
 // zero f where the scratch smooth (trilinear from the decimated grid) is below the cut,
-// the cut chosen by the local texture |orig - smooth| (pipeline.c:355-399)
-__global__ void __launch_bounds__(1024) k_air_apply(AirArgs a) {
-    __shared__ unsigned wbits[32];
-    const long x = (long)blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    const bool in = x < a.nx;
+// the cut chosen by the local texture |orig - smooth| (pipeline.c:355-399).
+//
+// Bound by issue and latency, not by memory (the fields of a tile live in L2): a warp takes a whole
+// row, so that everything of y and z is formed once per row, and walks it 32 voxels at a time. The
+// material bits come out of the walk's ballots, and with the run carried from word to word each
+// word's first voxel can point at its run's head in an earlier word: no barrier, and labels only at
+// run heads instead of at every voxel. Measured at 144^3:
+// 21.9 us against 31.8 with a CTA per row, which also wrote a label per voxel.
+__global__ void __launch_bounds__(32 * kRowWarps) k_air_apply(AirArgs a) {
+    const unsigned row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, nx = (int)a.nx;
+    if (row >= (unsigned)(a.nz * a.ny)) return;
+    const int z = (int)(row / (unsigned)a.ny), y = (int)(row - (unsigned)z * (unsigned)a.ny);
     const float cu = a.ctl->cutf_uni, ct = a.ctl->cutf_tex;
-    for (long z = blockIdx.z; z < a.nz; z += gridDim.z) {
-        const size_t i = ((size_t)z * a.ny + y) * a.nx + x;
-        float fv = 0.0f;
-        if (in) {
+    const int base = (int)(row * (unsigned)nx);
+    int z0 = z >> 1, y0 = y >> 1;
+    if (z0 > a.lz - 2) z0 = (int)a.lz - 2;
+    if (y0 > a.ly - 2) y0 = (int)a.ly - 2;
+    float zf = __fsub_rn(__fmul_rn(0.5f, (float)z), (float)z0), yf = __fsub_rn(__fmul_rn(0.5f, (float)y), (float)y0);
+    zf = zf > 1.0f ? 1.0f : zf;
+    yf = yf > 1.0f ? 1.0f : yf;
+    const float w00 = __fmul_rn(1.0f - zf, 1.0f - yf), w01 = __fmul_rn(1.0f - zf, yf);
+    const float w10 = __fmul_rn(zf, 1.0f - yf), w11 = __fmul_rn(zf, yf);
+    const int lx = (int)a.lx;
+    const float* s00 = a.sm + (a.lowres ? ((size_t)z0 * a.ly + y0) * lx : (size_t)base);
+    const float *s01 = s00 + lx, *s10 = s00 + (size_t)a.ly * lx, *s11 = s10 + lx;
+    int head = -1;                           // first voxel of the run that reaches the word's end, or -1
+    for (int w = 0; w * 32 < nx; ++w) {
+        const int x = w * 32 + lane;
+        bool mat = false;
+        if (x < nx) {
             float v;
             if (a.lowres) {
-                long z0 = z >> 1, y0 = y >> 1, x0 = x >> 1;
-                if (z0 > a.lz - 2) z0 = a.lz - 2;
-                if (y0 > a.ly - 2) y0 = a.ly - 2;
-                if (x0 > a.lx - 2) x0 = a.lx - 2;
-                float zf = __fsub_rn(__fmul_rn(0.5f, (float)z), (float)z0);
-                float yf = __fsub_rn(__fmul_rn(0.5f, (float)y), (float)y0);
+                int x0 = x >> 1;
+                if (x0 > lx - 2) x0 = lx - 2;
                 float fx = __fsub_rn(__fmul_rn(0.5f, (float)x), (float)x0);
-                zf = zf > 1.0f ? 1.0f : zf;
-                yf = yf > 1.0f ? 1.0f : yf;
                 fx = fx > 1.0f ? 1.0f : fx;
-                const float w00 = __fmul_rn(1.0f - zf, 1.0f - yf), w01 = __fmul_rn(1.0f - zf, yf);
-                const float w10 = __fmul_rn(zf, 1.0f - yf), w11 = __fmul_rn(zf, yf);
-                const size_t r00 = ((size_t)z0 * a.ly + y0) * a.lx, r01 = r00 + a.lx;
-                const size_t r10 = r00 + (size_t)a.ly * a.lx, r11 = r10 + a.lx;
-                const float a0 = blend4(a.sm, r00, r01, r10, r11, x0, w00, w01, w10, w11);
-                const float a1 = blend4(a.sm, r00, r01, r10, r11, x0 + 1, w00, w01, w10, w11);
+                const float a0 = blend4(s00[x0], s01[x0], s10[x0], s11[x0], w00, w01, w10, w11);
+                const float a1 = blend4(s00[x0 + 1], s01[x0 + 1], s10[x0 + 1], s11[x0 + 1], w00, w01, w10, w11);
                 v = __fmaf_rn(__fsub_rn(a1, a0), fx, a0);
             } else {
-                v = a.sm[i];
+                v = s00[x];
             }
-            const float o = a.orig[i];
-            const float tex = fabsf(__fsub_rn(o, v));
-            fv = a.f[i];
-            if (v < (tex < 0.03f ? cu : ct)) { fv = 0.0f; a.f[i] = 0.0f; }
+            const float tex = fabsf(__fsub_rn(a.orig[base + x], v));
+            const float fv = a.f[base + x];
+            const bool air = v < (tex < 0.03f ? cu : ct);
+            if (air) a.f[base + x] = 0.0f;
+            mat = !air && fv > 0.0f;
         }
-        if (a.lab) {               // despeckle on: each material voxel points at its x-run's first voxel
-            const bool mat = in && fv > 0.0f;
-            const int head = run_head(mat, wbits);
-            if (in) {
-                const int t = (int)threadIdx.x;
-                a.lab[i] = mat ? (int)(i - (size_t)(t - head)) : -1;
-                if (mat && t == head) a.info[i] = 0u;       // run heads are the only possible roots
+        if (a.mask) {
+            const unsigned bits = __ballot_sync(0xffffffffu, mat);
+            if (mat && (lane == 0 || !(bits >> (lane - 1) & 1u))) {
+                a.lab[base + x] = lane == 0 && head >= 0 ? head : base + x;
+                a.info[base + x] = 0u;
             }
+            if (lane == 0) a.mask[(size_t)row * a.words + w] = bits;
+            if (!(bits >> 31)) head = -1;
+            else if (~bits) head = base + w * 32 + 32 - __clz(~bits);
+            else if (head < 0) head = base + w * 32;
         }
     }
 }
@@ -561,79 +557,90 @@ __device__ __forceinline__ void uf_union(int* L, int a, int b, int* err) {
 }
 
 struct CcArgs {
-    float* f;
+    const unsigned* mask;
+    int words;
     int* lab;
     unsigned* info;
     int* err;
-    long nz, ny, nx;
+    int nz, ny, nx;
     int min_size;
 };
 
-// Join runs: across a row-segment (CTA) boundary in x, and to the -y and -z neighbours where
-// a run overlap starts (if the left neighbours are both material, they already joined the
-// runs). Launched with the air pass's CTA width, so the segments are the same.
-__global__ void __launch_bounds__(1024) k_cc_union(CcArgs a) {
-    const long x = (long)blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= a.nx) return;
-    const int nx = (int)a.nx, plane = (int)(a.ny * a.nx);
-    for (long z = blockIdx.z; z < a.nz; z += gridDim.z) {
-        const int i = (int)(((size_t)z * a.ny + y) * a.nx + x);
-        // Only the signs (material or not) are read here, and those never change; issuing
-        // all six loads before any test keeps them to one memory round trip.
-        const int c = a.lab[i];
-        const int l = x > 0 ? a.lab[i - 1] : -1;
-        const int u = y > 0 ? a.lab[i - nx] : -1;
-        const int ul = (x > 0 && y > 0) ? a.lab[i - 1 - nx] : -1;
-        const int d = z > 0 ? a.lab[i - plane] : -1;
-        const int dl = (x > 0 && z > 0) ? a.lab[i - 1 - plane] : -1;
-        if (c < 0) continue;
-        const bool left = l >= 0;
-        if (left && x % blockDim.x == 0) uf_union(a.lab, i, i - 1, a.err);   // across row segments
-        if (u >= 0 && !(left && ul >= 0)) uf_union(a.lab, i, i - nx, a.err);
-        if (d >= 0 && !(left && dl >= 0)) uf_union(a.lab, i, i - plane, a.err);
+// The nodes of the union-find are the x-runs of material within a word of 32 voxels, each named by
+// its first voxel; a run that enters a word from the left was linked to its head by the air pass.
+// The run of bit b of word c starts at:
+__device__ __forceinline__ int run_start(unsigned c, int b) {
+    const unsigned gaps = ~c & ((1u << b) - 1u);
+    return gaps ? 32 - __clz(gaps) : 0;
+}
+
+// Join runs to those of the -y (blockIdx.y = 0) and -z (1) neighbour rows, once per overlap: where
+// an overlap starts (if the left neighbours are both material, they already joined the runs). A
+// thread takes a word, so that a solid row costs five threads and one join instead of a test of six
+// labels at each of its voxels; what is left is the walks' latency. Measured at 144^3:
+// 35.7 us against 39.7. (Joining blocks of rows in shared memory first cost more than it took off this
+// pass: 29 us for the blocks, 9 to 20 us left here.)
+__global__ void __launch_bounds__(128) k_cc_union(CcArgs a) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (unsigned)a.nz * a.ny * a.words) return;
+    const unsigned row = t / (unsigned)a.words, w = t - row * (unsigned)a.words;
+    const unsigned z = row / (unsigned)a.ny, y = row - z * (unsigned)a.ny;
+    const unsigned back = blockIdx.y ? (unsigned)a.ny : 1u;          // rows to the neighbour
+    if (blockIdx.y ? z == 0 : y == 0) return;
+    const unsigned q = t - back * (unsigned)a.words;
+    const unsigned c = a.mask[t], u = a.mask[q], o = c & u;
+    if (!o) return;
+    const unsigned joined = w ? (a.mask[t - 1] & a.mask[q - 1]) >> 31 : 0u;
+    const int i = (int)(row * (unsigned)a.nx + w * 32u), j = i - (int)(back * (unsigned)a.nx);
+    for (unsigned s = o & ~(o << 1 | joined); s; s &= s - 1) {
+        const int b = __ffs(s) - 1;
+        uf_union(a.lab, i + run_start(c, b), j + run_start(u, b), a.err);
     }
 }
 
-// Roots by read-only walks from the x-run heads (a run's voxels share its head's root;
-// each thread then stores its voxel's root for the zero pass), component sizes and face
-// contact with one atomic per run of equal roots in a warp. A count stops growing once it
-// reaches min_size and a face-touching root takes no count: both leave the zero test
-// (no face contact and fewer than min_size voxels) unchanged.
-__global__ void __launch_bounds__(1024) k_cc_count(CcArgs a) {
-    __shared__ unsigned wbits[32];
-    __shared__ int sroot[1024];
-    const long x = (long)blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    const int lane = threadIdx.x & 31;
-    const bool in = x < a.nx;
-    for (long z = blockIdx.z; z < a.nz; z += gridDim.z) {
-        const size_t i = ((size_t)z * a.ny + y) * a.nx + x;
-        const int l = in ? __ldcg(a.lab + i) : -1;
-        // the voxel's x-run (within the CTA's row segment) shares one root: the head walks
-        const int head = run_head(l >= 0, wbits);
-        const int t = (int)threadIdx.x;
-        if (l >= 0 && t == head) sroot[t] = uf_root(a.lab, l, a.err);
-        __syncthreads();
-        const int root = l >= 0 ? sroot[head] : -1;
-        __syncthreads();                     // sroot is rewritten by the next row
-        if (root >= 0) a.lab[i] = root;
-        const bool edge = root >= 0 && (z == 0 || z == a.nz - 1 || y == 0 || y == a.ny - 1 || x == 0 || x == a.nx - 1);
-        const int prev = __shfl_up_sync(0xffffffffu, root, 1);
-        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != root);
-        const unsigned edges = __ballot_sync(0xffffffffu, edge);
-        if (root >= 0 && (lane == 0 || prev != root)) {
-            const unsigned after = heads & ~((2u << lane) - 1u);      // run heads above this lane
-            const int end = after ? __ffs(after) - 1 : 32;
-            const unsigned seg = (end == 32 ? 0xffffffffu : (1u << end) - 1u) & ~((1u << lane) - 1u);
-            // Only "touches a face" and "has at least min_size voxels" decide the zero pass, so
-            // a root already known to be either takes no more atomics (the giant components
-            // would otherwise serialise on one address).
-            const unsigned v = __ldcg(a.info + root);
-            if (!(v & kEdge)) {
-                if (edges & seg) atomicOr(&a.info[root], kEdge);
-                else if ((long)(v & ~kEdge) < a.min_size) atomicAdd(&a.info[root], (unsigned)(end - lane));
+// Roots by read-only walks from the nodes (stored for the quantiser), component sizes and face
+// contact. A count stops growing once it reaches min_size and a face-touching root takes no count:
+// both leave the zero test (no face contact and fewer than min_size voxels) unchanged, and a root
+// already known to be either takes no more atomics (the giant components would otherwise serialise
+// on one address). A thread takes a word and adds up its runs of one root; the last root of each
+// thread is added up over the warp. Measured at 144^3: 16.0 us against 29.1 with a thread per
+// voxel.
+__global__ void __launch_bounds__(128) k_cc_count(CcArgs a) {
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    auto put = [&](int root, unsigned n, unsigned edge) {
+        const unsigned v = __ldcg(a.info + root);
+        if (v & kEdge) return;
+        if (edge) atomicOr(&a.info[root], kEdge);
+        else if ((long)v < a.min_size) atomicAdd(&a.info[root], n);
+    };
+    int cur = -1;
+    unsigned n = 0, edge = 0;
+    if (t < (unsigned)a.nz * a.ny * a.words) {
+        const unsigned row = t / (unsigned)a.words, w = t - row * (unsigned)a.words;
+        const int z = (int)(row / (unsigned)a.ny), y = (int)(row - (unsigned)z * (unsigned)a.ny);
+        const bool face = z == 0 || z == a.nz - 1 || y == 0 || y == a.ny - 1;
+        const int i = (int)(row * (unsigned)a.nx + w * 32u);
+        unsigned c = a.mask[t];
+        while (c) {
+            const int b = __ffs(c) - 1;
+            const unsigned gaps = ~(c >> b);                         // shifted-in zeros are gaps
+            const int len = gaps ? __ffs(gaps) - 1 : 32;
+            c = b + len < 32 ? c & ~((1u << (b + len)) - 1u) : 0u;
+            const int root = uf_root(a.lab, i + b, a.err);
+            a.lab[i + b] = root;
+            const unsigned e = face || (w == 0 && b == 0) || (int)w * 32 + b + len == a.nx;
+            if (root != cur) {
+                if (cur >= 0) put(cur, n, edge);
+                cur = root; n = 0; edge = 0;
             }
+            n += len;
+            edge |= e;
         }
     }
+    const unsigned peers = __match_any_sync(0xffffffffu, cur);
+    n = __reduce_add_sync(peers, n);
+    edge = __reduce_or_sync(peers, edge);
+    if (cur >= 0 && __ffs(peers) - 1 == (int)(threadIdx.x & 31)) put(cur, n, edge);
 }
 
 // ---------------------------------------------------------------- recenter + quantise
@@ -646,22 +653,31 @@ struct QuantArgs {
     long gz0, gy0, gx0;       // inner tile origin in the volume
     int no_dither, norm;
     float midf, k;
-    const int* lab;           // despeckle on: voxel -> component root (k_cc_count), else nullptr
+    const unsigned* mask;     // despeckle on: material bits, else nullptr
+    int words;
+    const int* lab;           // run head -> component root (k_cc_count)
     const unsigned* info;
     int min_size;
 };
 
-__global__ void __launch_bounds__(1024) k_tile_quant(QuantArgs a) {
-    const long x = (long)blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x >= a.tx) return;
-    for (long z = blockIdx.z; z < a.tz; z += gridDim.z) {
-        const size_t j = ((size_t)(a.iz0 + z) * a.hy + (a.iy0 + y)) * a.hx + (a.ix0 + x);
-        float v = a.f[j];
-        if (a.lab) {                        // the despeckle's zeroing, for the voxels kept
-            const int root = a.lab[j];
-            if (root >= 0) {
-                const unsigned c = a.info[root];
-                if (!(c & kEdge) && (long)(c & ~kEdge) < a.min_size) v = 0.0f;
+// A warp per row of the inner tile. Measured at 128^3 inside 144^3: 12.6 us against 15.3 with a CTA per
+// row and a label per voxel.
+__global__ void __launch_bounds__(32 * kRowWarps) k_tile_quant(QuantArgs a) {
+    const unsigned row = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    if (row >= (unsigned)(a.tz * a.ty)) return;
+    const int z = (int)(row / (unsigned)a.ty), y = (int)(row - (unsigned)z * (unsigned)a.ty);
+    const size_t brow = (size_t)(a.iz0 + z) * a.hy + (a.iy0 + y);
+    const float* f = a.f + brow * a.hx + a.ix0;
+    const unsigned* mask = a.mask + (a.mask ? brow * a.words : 0);
+    uint8_t* out = a.out + (size_t)row * a.tx;
+    for (int x = (int)(threadIdx.x & 31); x < (int)a.tx; x += 32) {
+        float v = f[x];
+        if (a.mask) {                       // the despeckle's zeroing, for the voxels kept
+            const int bx = (int)a.ix0 + x, b = bx & 31;
+            const unsigned c = mask[bx >> 5];
+            if (c >> b & 1u) {
+                const unsigned m = a.info[a.lab[brow * a.hx + (bx - b) + run_start(c, b)]];
+                if (!(m & kEdge) && (long)m < a.min_size) v = 0.0f;
             }
         }
         if (a.norm) {
@@ -678,13 +694,13 @@ __global__ void __launch_bounds__(1024) k_tile_quant(QuantArgs a) {
             const int qi = (int)t;
             q = qi > 255 ? 255 : (uint8_t)qi;
         }
-        a.out[((size_t)z * a.ty + y) * a.tx + x] = q;
+        out[x] = q;
     }
 }
 
 // ---------------------------------------------------------------- host side
 struct TileWs {
-    fy::DevBuf u8, orig, work, alt, t1, t2, sm, lab, info, tab, ctl, out;
+    fy::DevBuf u8, orig, work, alt, t1, t2, sm, mask, lab, info, tab, ctl, out;
     fy::HostBuf pin, hin, hout;   // control and tables; host-API staging of the u8 tile in/out
     bool have_state = false;
     long hist[256];
@@ -697,13 +713,8 @@ unsigned grid1(size_t n, int tpb, int sms) {
     return (unsigned)std::max<size_t>(1, std::min(g, cap));
 }
 
-// Row kernels: a CTA spans a row (x) in whole warps, up to 1024 threads; grid (x, y, z).
-// Warp lanes stay aligned with x % 32, which the run labels rely on.
-int row_threads(long nx) { return (int)std::min<long>(1024, (nx + 31) / 32 * 32); }
-dim3 grid_rows(long nx, long ny, long nz) {
-    const long t = row_threads(nx);
-    return dim3((unsigned)((nx + t - 1) / t), (unsigned)ny, (unsigned)std::min<long>(nz, 65535));
-}
+// Row kernels: a warp per row.
+unsigned grid_rows(long ny, long nz) { return (unsigned)((ny * nz + kRowWarps - 1) / kRowWarps); }
 
 // eps_for_tile, pipeline.c:447-456
 double tile_eps(const fy_pipeline_cfg* c, double ecy, double ecx, long y0, long x0, long ty, long tx) {
@@ -885,21 +896,26 @@ int tile_chain(const fy_pipeline_cfg* c, const uint8_t* d_u8, long rz0, long ry0
         TRY(cudaGetLastError());
         fy_prof_mark(st, "tile.air_cut");
         const bool cc = c->air_min_component > 0;
+        const int words = (int)((hx + 31) / 32);
+        const size_t nwords = (size_t)hz * hy * words;
         if (cc) {
+            TRY(w.mask.ensure(nwords * sizeof(unsigned)));
             TRY(w.lab.ensure(hn * sizeof(int)));
             TRY(w.info.ensure(hn * sizeof(unsigned)));
         }
-        AirArgs aa{f, orig, sm, ctl, hz, hy, hx, lz, ly, lx, lowres ? 1 : 0, cc ? w.lab.as<int>() : nullptr,
-                   cc ? w.info.as<unsigned>() : nullptr};
-        k_air_apply<<<grid_rows(hx, hy, hz), row_threads(hx), 0, st>>>(aa);
+        AirArgs aa{f, orig, sm, ctl, hz, hy, hx, lz, ly, lx, lowres ? 1 : 0, cc ? w.mask.as<unsigned>() : nullptr,
+                   words, w.lab.as<int>(), w.info.as<unsigned>()};
+        k_air_apply<<<grid_rows(hy, hz), 32 * kRowWarps, 0, st>>>(aa);
         TRY(cudaGetLastError());
         launches += 5;
         fy_prof_mark(st, "tile.air_apply");
         if (cc) {
-            CcArgs ca{f, w.lab.as<int>(), w.info.as<unsigned>(), &ctl->err, hz, hy, hx, c->air_min_component};
-            k_cc_union<<<grid_rows(hx, hy, hz), row_threads(hx), 0, st>>>(ca);
+            CcArgs ca{w.mask.as<unsigned>(), words, w.lab.as<int>(), w.info.as<unsigned>(), &ctl->err,
+                      (int)hz, (int)hy, (int)hx, c->air_min_component};
+            const unsigned cg = (unsigned)((nwords + 127) / 128);
+            k_cc_union<<<dim3(cg, 2), 128, 0, st>>>(ca);
             fy_prof_mark(st, "tile.cc_union");
-            k_cc_count<<<grid_rows(hx, hy, hz), row_threads(hx), 0, st>>>(ca);
+            k_cc_count<<<cg, 128, 0, st>>>(ca);
             TRY(cudaGetLastError());
             launches += 2;
             fy_prof_mark(st, "tile.cc_count");
@@ -919,11 +935,13 @@ int tile_chain(const fy_pipeline_cfg* c, const uint8_t* d_u8, long rz0, long ry0
         q.midf = 0.5f * (float)(c->norm_lo + c->norm_hi) * (1.0f / 255.0f);
         q.k = q.norm ? (2.0f * 0.375f) * 255.0f / (float)(c->norm_hi - c->norm_lo) : 0.0f;
         const bool cc = c->do_air_zero && c->air_min_component > 0;
-        q.lab = cc ? w.lab.as<int>() : nullptr;
-        q.info = cc ? w.info.as<unsigned>() : nullptr;
+        q.mask = cc ? w.mask.as<unsigned>() : nullptr;
+        q.words = (int)((hx + 31) / 32);
+        q.lab = w.lab.as<int>();
+        q.info = w.info.as<unsigned>();
         q.min_size = c->air_min_component;
         if (tn) {
-            k_tile_quant<<<grid_rows(tx, ty, tz), row_threads(tx), 0, st>>>(q);
+            k_tile_quant<<<grid_rows(ty, tz), 32 * kRowWarps, 0, st>>>(q);
             TRY(cudaGetLastError());
             launches++;
         }
@@ -1024,7 +1042,7 @@ extern "C" int fy_process_buffer(const fy_pipeline_cfg* cfg, const unsigned char
 
 void fy_tile_release() {
     TileWs& w = tws;
-    for (fy::DevBuf* b : {&w.u8, &w.orig, &w.work, &w.alt, &w.t1, &w.t2, &w.sm, &w.lab, &w.info, &w.tab, &w.ctl, &w.out})
+    for (fy::DevBuf* b : {&w.u8, &w.orig, &w.work, &w.alt, &w.t1, &w.t2, &w.sm, &w.mask, &w.lab, &w.info, &w.tab, &w.ctl, &w.out})
         b->release();
     w.pin.release();
     w.hin.release();

@@ -152,38 +152,50 @@ __global__ void k_decimate(const float* __restrict__ in, float* __restrict__ lo,
 // out = a*I + b with a, b trilinear from the low grid (guided.c:188-228): low sample i sits
 // at full coordinate i*s; u = (float)x/s, i0 = min((int)u, l-2), f = min(u - i0, 1); the
 // four (z,y) rows are blended with w00..w11 first, then lerped in x.
-__global__ void __launch_bounds__(256) k_upsample_apply(const float* __restrict__ in, float* __restrict__ out,
-                                                        const float* __restrict__ ma, const float* __restrict__ mb,
-                                                        int nz, int ny, int nx, int lz, int ly, int lx, int s) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y, z = blockIdx.z;
-    if (x >= nx) return;
-    const float fs = (float)s;
+// Bound by issue, not by memory: a warp takes a whole row, so that z, y, their weights and the four
+// coefficient rows are formed once per row instead of at every voxel, and x / s is a product where
+// 1 / s is exact (s a power of two; a division otherwise, with the same bits either way). Measured at
+// 144^3, s = 2: 20.3 us against 22.0 with a CTA per row.
+constexpr int kUpRows = 8;               // rows (warps) of a CTA
+__global__ void __launch_bounds__(32 * kUpRows) k_upsample_apply(const float* __restrict__ in, float* __restrict__ out,
+                                                                 const float* __restrict__ ma,
+                                                                 const float* __restrict__ mb, int nz, int ny, int nx,
+                                                                 int lz, int ly, int lx, int s) {
+    const size_t row = (size_t)blockIdx.x * kUpRows + (threadIdx.x >> 5);
+    if (row >= (size_t)nz * ny) return;
+    const int z = (int)(row / (unsigned)ny), y = (int)(row - (size_t)z * ny);
+    const float fs = (float)s, is = 1.0f / fs;
+    const bool exact = (s & (s - 1)) == 0;
     const float uz = (float)z / fs;
     int z0 = (int)uz; if (z0 > lz - 2) z0 = lz - 2;
     float zf = uz - z0; if (zf > 1.0f) zf = 1.0f;
     const float uy = (float)y / fs;
     int y0 = (int)uy; if (y0 > ly - 2) y0 = ly - 2;
     float yfr = uy - y0; if (yfr > 1.0f) yfr = 1.0f;
-    const float ux = (float)x / fs;
-    int x0 = (int)ux; if (x0 > lx - 2) x0 = lx - 2;
-    float fx = ux - x0; if (fx > 1.0f) fx = 1.0f;
-    const float gx = 1 - fx;
-    const size_t r00 = ((size_t)z0 * ly + y0) * lx, r01 = r00 + lx;
-    const size_t r10 = r00 + (size_t)ly * lx, r11 = r10 + lx;
+    const size_t r00 = ((size_t)z0 * ly + y0) * lx, r10 = r00 + (size_t)ly * lx;
+    const float *a00 = ma + r00, *a01 = a00 + lx, *a10 = ma + r10, *a11 = a10 + lx;
+    const float *b00 = mb + r00, *b01 = b00 + lx, *b10 = mb + r10, *b11 = b10 + lx;
     const float w00 = (1 - zf) * (1 - yfr), w01 = (1 - zf) * yfr;
     const float w10 = zf * (1 - yfr), w11 = zf * yfr;
-    float ar[2], br[2];
+    const float* pi = in + row * nx;
+    float* po = out + row * nx;
+#pragma unroll 2
+    for (int x = (int)(threadIdx.x & 31); x < nx; x += 32) {
+        const float ux = exact ? (float)x * is : (float)x / fs;
+        int x0 = (int)ux; if (x0 > lx - 2) x0 = lx - 2;
+        float fx = ux - x0; if (fx > 1.0f) fx = 1.0f;
+        const float gx = 1 - fx;
+        float ar[2], br[2];
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int k = x0 + q;
-        ar[q] = w00 * __ldg(ma + r00 + k) + w01 * __ldg(ma + r01 + k) + w10 * __ldg(ma + r10 + k) + w11 * __ldg(ma + r11 + k);
-        br[q] = w00 * __ldg(mb + r00 + k) + w01 * __ldg(mb + r01 + k) + w10 * __ldg(mb + r10 + k) + w11 * __ldg(mb + r11 + k);
+        for (int q = 0; q < 2; ++q) {
+            const int k = x0 + q;
+            ar[q] = w00 * __ldg(a00 + k) + w01 * __ldg(a01 + k) + w10 * __ldg(a10 + k) + w11 * __ldg(a11 + k);
+            br[q] = w00 * __ldg(b00 + k) + w01 * __ldg(b01 + k) + w10 * __ldg(b10 + k) + w11 * __ldg(b11 + k);
+        }
+        const float a = gx * ar[0] + fx * ar[1];
+        const float b = gx * br[0] + fx * br[1];
+        po[x] = a * pi[x] + b;
     }
-    const float a = gx * ar[0] + fx * ar[1];
-    const float b = gx * br[0] + fx * br[1];
-    const size_t i = ((size_t)z * ny + y) * nx + x;
-    out[i] = a * in[i] + b;
 }
 }  // namespace
 
@@ -204,9 +216,8 @@ cudaError_t fy_launch_guided_fast(const float* in, float* out, float* ws, int nz
     k_decimate<<<grid_1d(nl), 256, 0, st>>>(in, il, ny, nx, lz, ly, lx, fy_pitch(lx), s);
     cudaError_t e = fy_launch_guided_fused(il, ma, mb, ab, lz, ly, lx, rl, eps, 1, sms, st, eps_ptr, nullptr, fy_pitch(lx));
     if (e != cudaSuccess) return e;
-    const int tpb = nx < 256 ? (nx + 31) / 32 * 32 : 256;     // whole warps across a row
-    dim3 grid(ceil_div_i(nx, tpb), ny, nz);
-    k_upsample_apply<<<grid, tpb, 0, st>>>(in, out, ma, mb, nz, ny, nx, lz, ly, lx, s);
+    const unsigned grid = (unsigned)(((size_t)nz * ny + kUpRows - 1) / kUpRows);
+    k_upsample_apply<<<grid, 32 * kUpRows, 0, st>>>(in, out, ma, mb, nz, ny, nx, lz, ly, lx, s);
     launches += 4;
     return cudaGetLastError();
 }

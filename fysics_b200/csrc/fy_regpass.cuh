@@ -1,6 +1,7 @@
 // fy_regpass.cuh -- the deconvolution's five passes for axis lengths with a register plan
 // (fy_regfft.cuh).
 #pragma once
+#include <limits.h>
 #include "fy_internal.h"
 #include "fy_regfft.cuh"
 
@@ -28,15 +29,21 @@ template <int N> struct Col {
 // (plane p, stride pstride). The last one, kx = px/2, would cost a tile of its own per row with
 // one column in W used (11% of the tiles at px = 256); instead W rows' last columns share a tile.
 // Those tiles come first: their loads are 16 rows apart instead of one run and take longest.
+// They take several times a regular tile's time (16 sectors a request), so they are made only where
+// at least `least` regular tiles hide them; below that the partly filled tiles are faster. Measured
+// (us, shared against own): Y at 16 x 384^2 26.8 / 10.3, 16 x 512^2 22.5 / 12.3, 64^3 8.2 / 6.3, 192^3
+// 16.4 / 13.3, 256^3 26.6 / 28.6, 384^3 112.6 / 107, 512^3 190 / 179; Z at 128^3 14.3 / 12.3, 192^3
+// 20.5 / 22.5, 256^3 36.9 / 38.9, 384^3 186 / 201, 512^3 305 / 311. So a Y pass shares them from two
+// waves of CTAs on up to 256 points (above, a tile of its own is under 5% more work), a Z pass from one.
 struct ColTiles {
     int regular;              // tiles per row over the kx < px/2 columns (or over all hx columns)
     int rows;                 // rows (planes of a Y pass, y of a Z pass)
     unsigned last, total;     // tiles of last columns, tiles in all
     FastDiv dreg;
 };
-inline ColTiles col_tiles(int hx, int rows, int W) {
+inline ColTiles col_tiles(int hx, int rows, int W, long least = 0) {
     ColTiles c;
-    const bool split = hx > 1 && (hx - 1) % W == 0;
+    const bool split = hx > 1 && (hx - 1) % W == 0 && (long)((hx - 1) / W) * rows >= least;
     c.regular = split ? (hx - 1) / W : (hx + W - 1) / W;
     c.rows = rows;
     c.dreg = FastDiv((uint32_t)c.regular);
@@ -342,7 +349,7 @@ template <int N>
 inline cudaError_t launch_y(float2* spec, const SpecGeom& g, const float2* tw, int nplanes, int sign, int keep_rows,
                             cudaStream_t st) {
     using C = Col<N>;
-    const ColTiles ct = col_tiles(g.hx, nplanes, C::W);
+    const ColTiles ct = col_tiles(g.hx, nplanes, C::W, N <= 256 ? 2 * 148L * C::minb : LONG_MAX);
     if (sign > 0) return launch(k_col_y<N, 1, false>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, keep_rows);
     if (g.ny == N) return launch(k_col_y<N, -1, false>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, N);
     return launch(k_col_y<N, -1, true>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, g.ny, N);
@@ -368,7 +375,7 @@ cudaError_t deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
     case 4: return launch_y<N>(d.spec, g, d.twy, g.nz, +1, g.ny, st);
     case 3: {
         using C = Col<N>;
-        const ColTiles ct = col_tiles(g.hx, g.py, C::W);
+        const ColTiles ct = col_tiles(g.hx, g.py, C::W, 148L * C::minb);
         if (g.nz == N)
             return launch(k_col_z<N, false>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);
         return launch(k_col_z<N, true>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);

@@ -11,7 +11,7 @@ namespace rf {
 // A CTA transforms W = 16 columns, one 128-byte run per point, with TPL threads a column, the
 // column index fastest. Its tile crosses shared memory once per transform, stored point-major
 // (s[i*W + l]: a half warp's 16 columns are 16 consecutive float2, no conflicts).
-// What bounds them: HBM at 512 (the Y passes move 1.07 GB in 190 us, 0.86 of the measured copy
+// What bounds them: HBM at 512 (the Y passes move 1.07 GB in 180 us, 0.91 of the measured copy
 // rate), latency below. Sixteen warps an SM with 128 registers and no spills: at 512^3 the Z pass
 // takes 307 us so, 379 us with 8-column tiles (64-byte runs) and 20 warps, 434 us with 24 warps at
 // 80 registers (spills, and more tiles in flight than HBM serves well). The shared-memory passes

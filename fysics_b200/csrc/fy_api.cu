@@ -6,6 +6,7 @@
 // their contract is the reference's synchronous one.
 #include <math.h>
 #include <string.h>
+#include <cmath>
 #include <vector>
 
 #include "fy_context.h"
@@ -198,6 +199,12 @@ size_t fy_deconv_table_bytes(const SpecGeom& g) {
     const size_t lut_bytes = ((FY_LUT_N + 1) * sizeof(float) + 15) & ~(size_t)15;
     return lut_bytes + sizeof(double) * ((size_t)g.pz + g.py + g.hx);
 }
+// The largest u = f^2 of the padded grid (the f of every axis is largest at its middle), which the
+// table's last entry stands for.
+static double table_umax(const SpecGeom& g, double fz2s) {
+    const double fz = (double)(g.pz / 2) / g.pz, fy = (double)(g.py / 2) / g.py, fx = (double)(g.px / 2) / g.px;
+    return fz * fz * fz2s + fy * fy + fx * fx;
+}
 double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double param, int kind, double fz2s,
                              void* host) {
     const size_t lut_bytes = ((FY_LUT_N + 1) * sizeof(float) + 15) & ~(size_t)15;
@@ -206,20 +213,19 @@ double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double para
     double* fz2 = (double*)(h + lut_bytes);
     double* fy2 = fz2 + g.pz;
     double* fx2 = fy2 + g.py;
-    double mz = 0, my = 0, mx = 0;
     for (int i = 0; i < g.pz; i++) {
         const double f = (i <= g.pz / 2) ? (double)i / g.pz : (double)(i - g.pz) / g.pz;
-        fz2[i] = f * f * fz2s; if (fz2[i] > mz) mz = fz2[i];
+        fz2[i] = f * f * fz2s;
     }
     for (int i = 0; i < g.py; i++) {
         const double f = (i <= g.py / 2) ? (double)i / g.py : (double)(i - g.py) / g.py;
-        fy2[i] = f * f; if (fy2[i] > my) my = fy2[i];
+        fy2[i] = f * f;
     }
     for (int i = 0; i < g.hx; i++) {
         const double f = (double)i / g.px;
-        fx2[i] = f * f; if (fx2[i] > mx) mx = fx2[i];
+        fx2[i] = f * f;
     }
-    const double umax = mz + my + mx;
+    const double umax = table_umax(g, fz2s);
     // A 1x1x1 volume has umax = 0; every sample then sits at u = 0 (us = 0 -> t = 0).
     const double us = umax > 0 ? FY_LUT_N / umax : 0.0;
     const double cap = kind == 1 ? 0.0 : FY_MAX_DECONV_GAIN;
@@ -302,6 +308,16 @@ void deconv_defaults(const fy_physics* p, int kind, double& param, double& fz2s)
     }
 }
 
+// A z scale with which the weight table has no finite scale (NaN, infinite, (sigma_z/sigma_xy)^2 too
+// large for a double, or so small that FY_LUT_N / umax overflows) gives no position in the table: the
+// reference indexes it with (int)NaN there and crashes. fz2s after deconv_defaults.
+int check_scale(const SpecGeom& g, double fz2s, const char* what) {
+    const double umax = table_umax(g, fz2s);
+    if (!std::isfinite(fz2s) || !std::isfinite(umax) || (umax > 0 && !std::isfinite(FY_LUT_N / umax)))
+        return fail(FY_EINVAL, "%s: z scale %g of the deconvolution's frequencies is not usable", what, fz2s);
+    return FY_OK;
+}
+
 // Enqueue the full deconvolution on st. src is device memory (u8 or f32), dst device f32.
 int enqueue_deconv(const void* src, int src_u8, double fmin, double fmax, float* dst, int dpitch, int nz, int ny,
                    int nx, const fy_physics* p, double param, int kind, double fz2s, cudaStream_t st,
@@ -311,6 +327,7 @@ int enqueue_deconv(const void* src, int src_u8, double fmin, double fmax, float*
     int rc = make_geom(nz, ny, nx, d.g, what);
     if (rc) return rc;
     deconv_defaults(p, kind, param, fz2s);
+    if ((rc = check_scale(d.g, fz2s, what))) return rc;
     d.plx = fy_make_plan(d.g.px); d.ply = fy_make_plan(d.g.py); d.plz = fy_make_plan(d.g.pz);
     d.twx = fy::twiddles(d.g.px); d.twy = fy::twiddles(d.g.py); d.twz = fy::twiddles(d.g.pz);
     if (!d.twx || !d.twy || !d.twz) return fail(FY_ENOMEM, "%s: twiddle tables", what);
@@ -325,11 +342,24 @@ int enqueue_deconv(const void* src, int src_u8, double fmin, double fmax, float*
     return FY_OK;
 }
 
+}  // namespace
+
+// Whether a deconvolution of this volume can run: its dims and, for the kind, its z scale. Callers
+// that do other work first ask before it.
+int fy_deconv_check(int nz, int ny, int nx, const fy_physics* p, int kind, double fz2s, const char* what) {
+    SpecGeom g;
+    const int rc = make_geom(nz, ny, nx, g, what);
+    if (rc) return rc;
+    double param = 1.0;
+    deconv_defaults(p, kind, param, fz2s);
+    return check_scale(g, fz2s, what);
+}
+
+namespace {
 int host_deconv(const float* in, float* out, int nz, int ny, int nx, const fy_physics* p, double param,
                 int kind, double fz2s, const char* what) {
     if (!in || !out || !p) return fail(FY_EINVAL, "%s: null pointer", what);
-    SpecGeom g;
-    int rc = make_geom(nz, ny, nx, g, what);
+    int rc = fy_deconv_check(nz, ny, nx, p, kind, fz2s, what);
     if (rc) return rc;
     if ((rc = fy::ensure_ctx())) return rc;
     fy::ThreadCtx& c = ctx();
@@ -358,6 +388,7 @@ int fy_deconv_setup(int nz, int ny, int nx, const fy_physics* p, double& param, 
     int rc = make_geom(nz, ny, nx, d.g, what);
     if (rc) return rc;
     deconv_defaults(p, kind, param, fz2s);
+    if ((rc = check_scale(d.g, fz2s, what))) return rc;
     d.plx = fy_make_plan(d.g.px); d.ply = fy_make_plan(d.g.py); d.plz = fy_make_plan(d.g.pz);
     d.twx = fy::twiddles(d.g.px); d.twy = fy::twiddles(d.g.py); d.twz = fy::twiddles(d.g.pz);
     if (!d.twx || !d.twy || !d.twz) return fail(FY_ENOMEM, "%s: twiddle tables", what);
@@ -407,8 +438,8 @@ extern "C" int fy_gpu_deconvolve_ex(const void* d_in, int src_u8, double f32_min
 int fy_deconvolve_pitched(const void* d_in, int src_u8, double f32_min, double f32_max, float* d_out, int dpitch, int nz,
                           int ny, int nx, const fy_physics* p, double param, int kind, double fz2_scale, cudaStream_t st) {
     if (kind < 0 || kind > 2) return fail(FY_EINVAL, "fy_gpu_deconvolve_ex: kind %d", kind);
-    int rc = fy::ensure_ctx();
-    if (rc) return rc;
+    int rc = fy_deconv_check(nz, ny, nx, p, kind, fz2_scale, "fy_gpu_deconvolve_ex");
+    if (rc || (rc = fy::ensure_ctx())) return rc;
     fy::ws_acquire(st);
     rc = enqueue_deconv(d_in, src_u8 ? 1 : 0, f32_min, f32_max, d_out, dpitch, nz, ny, nx, p, param, kind,
                         fz2_scale, st, "fy_gpu_deconvolve_ex");

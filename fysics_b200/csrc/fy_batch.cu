@@ -74,6 +74,8 @@ extern "C" int fy_gpu_restore_u8_batch(const fy_batch_cube* cubes, int n, const 
         const fy_batch_cube& q = cubes[i];
         if (!q.u8 || !q.out) return fail(FY_EINVAL, "%s: volume %d: null pointer", what, i);
         if (q.nz < 1 || q.ny < 1 || q.nx < 1) return fail(FY_EINVAL, "%s: volume %d: bad dims", what, i);
+        const int ok = fy_deconv_check(q.nz, q.ny, q.nx, &q.phys, cfg->deconv_kind, cfg->fz2_scale, what);
+        if (ok) return ok;
     }
     if (n == 0) return FY_OK;
     int rc = fy::ensure_ctx();

@@ -293,8 +293,7 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_z_weight(float2* __restrict__ 
                     const float2 v = s[i * W + ln.l];
                     const double2 yx = syx[ln.l];
                     const double t = ((sfz[i] + yx.x) + yx.y) * us;  // paganin.c:234-236
-                    int ti = (int)t;
-                    if (ti >= FY_LUT_N) ti = FY_LUT_N - 1;
+                    const int ti = (int)min((unsigned)(int)t, (unsigned)(FY_LUT_N - 1));
                     // the table (16 KB, read-only) through L1 rather than copied per tile
                     const float l0 = __ldg(lut + ti), l1 = __ldg(lut + ti + 1);
                     const float w = l0 + (l1 - l0) * (float)(t - ti);

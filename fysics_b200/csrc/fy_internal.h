@@ -35,6 +35,7 @@ size_t fy_deconv_spec_elems(const SpecGeom& g);
 // LUT index scale), their size, and the launch fields other than its buffers.
 size_t fy_deconv_table_bytes(const SpecGeom& g);
 double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double param, int kind, double fz2s, void* host);
+int fy_deconv_check(int nz, int ny, int nx, const fy_physics* p, int kind, double fz2s, const char* what);
 int fy_deconv_setup(int nz, int ny, int nx, const fy_physics* p, double& param, int kind, double& fz2s,
                     double fmin, double fmax, DeconvLaunch& d, const char* what);
 // fy_gpu_deconvolve_ex with output rows dpitch floats apart.

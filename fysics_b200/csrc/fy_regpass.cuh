@@ -157,7 +157,7 @@ k_col_z(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ ColTiles 
 #pragma unroll
     for (int m = 0; m < elems(N); ++m) {
         const double p = __dadd_rz(fma(__ldg(fz2 + t + tpl(N) * m), use, pyx), 0x1p20);
-        const float* cell = lut + (__double2hiint(p) - 0x41300000);
+        const float* cell = lut + min((unsigned)(__double2hiint(p) - 0x41300000), (unsigned)(FY_LUT_N - 1));
         const float l0 = __ldg(cell), l1 = __ldg(cell + 1);
         const float w = l0 + (l1 - l0) * (__uint2float_rn((unsigned)__double2loint(p)) * 0x1p-32f);
         v[m] = make_float2(v[m].x * w, v[m].y * w);

@@ -50,8 +50,8 @@ extern "C" int fy_gpu_restore_u8(const unsigned char* d_u8, float* d_out, int nz
     if (win / 2 > 4) return fail(FY_EUNSUPPORTED, "%s: noise win > 9", what);
     int radius = cfg->guided_radius < 1 ? 2 : cfg->guided_radius;
     if (radius > 4 && cfg->guided_s <= 1) return fail(FY_EUNSUPPORTED, "%s: chained guided radius > 4", what);
-    int rc = fy::ensure_ctx();
-    if (rc) return rc;
+    int rc = fy_deconv_check(nz, ny, nx, p, cfg->deconv_kind, cfg->fz2_scale, what);
+    if (rc || (rc = fy::ensure_ctx())) return rc;
     fy::ThreadCtx& c = ctx();
     cudaStream_t st = (cudaStream_t)stream;
     const size_t n = (size_t)nz * ny * nx;

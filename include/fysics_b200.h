@@ -277,6 +277,9 @@ int fy_gpu_phys_to_u8(const float *d_in, unsigned char *d_out, size_t n,
  *       2 = Paganin x unsharp Wiener with anisotropic z: fz^2 scaled by fz2_scale
  *           (= (sigma_z/sigma_xy)^2), cap 8, param = reg -- deconv_radial's fz2_scale
  *           (paganin.c:140-154), which fysics reaches only through the matched weight.
+ * A z scale with which the weight table has no finite scale (fz2_scale or, for kind 1,
+ * (psf_sigma_z_vox/psf_sigma_vox)^2: NaN, infinite, overflowing) returns FY_EINVAL, here and in
+ * every call that deconvolves.
  * src_u8 != 0: d_in is u8 and is dewindowed on load as fy_u8_to_phys(f32_min, f32_max). */
 int fy_gpu_deconvolve_ex(const void *d_in, int src_u8, double f32_min, double f32_max,
                          float *d_out, int nz, int ny, int nx, const fy_physics *p,

@@ -87,6 +87,8 @@ inline void count_launch(int k = 1) { ctx().launches += k; }
 inline void enter() { ThreadCtx& c = ctx(); c.status = 0; if (!c.err.empty()) c.err.clear(); }
 // Is `p` host memory that the GPU can DMA directly (pinned / registered)?
 bool is_pinned(const void* p);
+// Is `p` plain host memory, unknown to CUDA? (Anything else may not be the CPU's to read.)
+bool is_pageable(const void* p);
 // Is `p` device memory (or managed memory)?
 bool is_device(const void* p);
 

@@ -8,7 +8,8 @@
 // One fy_deconvolve after another on an 8x512x512 slab: 1300 -> 715 us (three helpers 797, seven 784;
 // smaller chunks cost more calls than they overlap); on 256^3 floats 10.2 -> 5.0 ms. Helpers live for one
 // call and are joined in it; all callers together have at most half the cores as helpers, and with
-// none (or no pinned memory, or a pinned caller) the plain copies run.
+// none (or no pinned memory, or a caller's buffer that is not pageable host memory: pinned, managed, on a
+// device) the plain copies run.
 #pragma once
 #include <string.h>
 #include <atomic>
@@ -47,7 +48,7 @@ public:
     HostCopy(const HostCopy&) = delete;
 
     cudaError_t to_device(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-        if (!stage_ || is_pinned(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+        if (!stage_ || !is_pageable(src)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
         char* ring = (char*)ctx().pin2.p;
         for (size_t at = 0; at < bytes; at += kRing) {
             const size_t n = bytes - at < kRing ? bytes - at : kRing;
@@ -67,7 +68,7 @@ public:
     }
     // Returns with the data in dst (the stream is waited for).
     cudaError_t from_device(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-        if (!stage_ || is_pinned(dst)) {
+        if (!stage_ || !is_pageable(dst)) {
             const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
             return e != cudaSuccess ? e : cudaStreamSynchronize(st);
         }

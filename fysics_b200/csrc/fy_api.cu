@@ -194,9 +194,9 @@ struct DeconvKey {
 
 // Plan-time tables of deconv_radial (paganin.c:213-230) into host memory of
 // fy_deconv_table_bytes(g) bytes: the 4097-entry float LUT of the capped weight over u = f^2
-// (padded to 16 bytes), then fz2, fy2 and fx2 in double. Returns the LUT index scale us.
+// and its last entry once more (16-byte aligned), then fz2, fy2 and fx2 in double. Returns the LUT index scale us.
 size_t fy_deconv_table_bytes(const SpecGeom& g) {
-    const size_t lut_bytes = ((FY_LUT_N + 1) * sizeof(float) + 15) & ~(size_t)15;
+    const size_t lut_bytes = fy_deconv_lut_bytes();
     return lut_bytes + sizeof(double) * ((size_t)g.pz + g.py + g.hx);
 }
 // The largest u = f^2 of the padded grid (the f of every axis is largest at its middle), which the
@@ -207,7 +207,7 @@ static double table_umax(const SpecGeom& g, double fz2s) {
 }
 double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double param, int kind, double fz2s,
                              void* host) {
-    const size_t lut_bytes = ((FY_LUT_N + 1) * sizeof(float) + 15) & ~(size_t)15;
+    const size_t lut_bytes = fy_deconv_lut_bytes();
     unsigned char* h = (unsigned char*)host;
     float* lut = (float*)h;
     double* fz2 = (double*)(h + lut_bytes);
@@ -235,6 +235,7 @@ double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double para
         if (cap > 0 && w > cap) w = cap;
         lut[i] = (float)w;
     }
+    lut[FY_LUT_N + 1] = lut[FY_LUT_N];
     return us;
 }
 
@@ -247,7 +248,7 @@ int deconv_tables(const SpecGeom& g, const fy_physics* p, double param, int kind
     memset(&key, 0, sizeof key);
     key.nz = g.nz; key.ny = g.ny; key.nx = g.nx; key.kind = kind;
     key.param = param; key.fz2s = fz2s; key.p = *p;
-    const size_t lut_bytes = ((FY_LUT_N + 1) * sizeof(float) + 15) & ~(size_t)15;
+    const size_t lut_bytes = fy_deconv_lut_bytes();
     const size_t bytes = fy_deconv_table_bytes(g);
     if (!(c.tab.valid && c.tab.keylen == sizeof key && !memcmp(c.tab.key, &key, sizeof key))) {
         std::vector<unsigned char> h(bytes);
@@ -404,7 +405,7 @@ int fy_deconv_reserve(int nz, int ny, int nx) {
     if (rc) return rc;
     if ((rc = fy::ensure_ctx())) return rc;
     fy::ThreadCtx& c = ctx();
-    const size_t lut_bytes = ((FY_LUT_N + 1) * sizeof(float) + 15) & ~(size_t)15;
+    const size_t lut_bytes = fy_deconv_lut_bytes();
     cudaError_t e;
     if ((e = c.spec.ensure(fy_deconv_spec_elems(g) * sizeof(float2))) != cudaSuccess ||
         (e = c.tab.buf.ensure(lut_bytes + sizeof(double) * ((size_t)g.pz + g.py + g.hx))) != cudaSuccess ||

@@ -150,7 +150,7 @@ extern "C" int fy_gpu_restore_u8_batch(const fy_batch_cube* cubes, int n, const 
     unsigned char* H = (unsigned char*)c.batch_pin.p;
     unsigned char* D = c.batch_up.as<unsigned char>();
     memset(H, 0, off_packs);                              // the queue counters start at 0
-    const size_t lut_bytes = ((FY_LUT_N + 1) * sizeof(float) + 15) & ~(size_t)15;
+    const size_t lut_bytes = fy_deconv_lut_bytes();
     fyzb::BoxJob* js = reinterpret_cast<fyzb::BoxJob*>(H + off_jobs_s);
     fyzb::BoxJob* jg = reinterpret_cast<fyzb::BoxJob*>(H + off_jobs_g);
     long long total_s = 0, total_g = 0;

@@ -33,6 +33,7 @@ cudaError_t fy_deconv_pass_ct_c(int pass, int n, const DeconvLaunch& d, cudaStre
 size_t fy_deconv_spec_elems(const SpecGeom& g);
 // Host side of a deconvolution (fy_api.cu): the plan-time tables into host memory (returns the
 // LUT index scale), their size, and the launch fields other than its buffers.
+constexpr size_t fy_deconv_lut_bytes() { return ((FY_LUT_N + 2) * sizeof(float) + 15) & ~(size_t)15; }
 size_t fy_deconv_table_bytes(const SpecGeom& g);
 double fy_deconv_fill_tables(const SpecGeom& g, const fy_physics* p, double param, int kind, double fz2s, void* host);
 int fy_deconv_check(int nz, int ny, int nx, const fy_physics* p, int kind, double fz2s, const char* what);

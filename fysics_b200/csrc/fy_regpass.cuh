@@ -148,18 +148,16 @@ k_col_z(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ ColTiles 
     load_tail_twiddles<N>(s + Col<N>::tile, tw);
     col_fft<N, -1>(v, s, l, t);
     asm volatile("" : "+l"(fz2), "+l"(lut));             // nor are the weights' loads moved before it
-    // Table position p = (fz^2 + fy^2 + fx^2)*us of paganin.c:234-236 in FP64; adding 2^20 towards
-    // zero leaves its integer part in the high word and its fraction's 32 bits in the low word.
-    // The last point of the table, p = 4096, would be cell 4096: us is taken 2^-33 smaller, which
-    // moves it to the end of cell 4095 (and a fraction by less than 2^-21).
-    const double use = us - us * 0x1p-33;
-    const double pyx = c.valid ? (__ldg(fy2 + c.row) + __ldg(fx2 + c.kx)) * use : 0.0;
+    // Table position p = (fz^2 + fy^2 + fx^2)*us of paganin.c:234-236, and its fraction, in FP64;
+    // adding 2^52 towards zero leaves the integer part in the low word. The last point of the table,
+    // p = 4096, is cell 4096, which the table continues with an equal entry.
+    const double pyx = c.valid ? (__ldg(fy2 + c.row) + __ldg(fx2 + c.kx)) * us : 0.0;
 #pragma unroll
     for (int m = 0; m < elems(N); ++m) {
-        const double p = __dadd_rz(fma(__ldg(fz2 + t + tpl(N) * m), use, pyx), 0x1p20);
-        const float* cell = lut + min((unsigned)(__double2hiint(p) - 0x41300000), (unsigned)(FY_LUT_N - 1));
+        const double p = fma(__ldg(fz2 + t + tpl(N) * m), us, pyx), ip = __dadd_rz(p, 0x1p52);
+        const float* cell = lut + min((unsigned)__double2loint(ip), (unsigned)FY_LUT_N);
         const float l0 = __ldg(cell), l1 = __ldg(cell + 1);
-        const float w = l0 + (l1 - l0) * (__uint2float_rn((unsigned)__double2loint(p)) * 0x1p-32f);
+        const float w = l0 + (l1 - l0) * (float)(p - (ip - 0x1p52));
         v[m] = make_float2(v[m].x * w, v[m].y * w);
     }
     __syncthreads();                                     // every thread has read the forward exchange

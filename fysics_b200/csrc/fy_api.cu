@@ -369,7 +369,7 @@ int host_deconv(const float* in, float* out, int nz, int ny, int nx, const fy_ph
     fy::ws_acquire(st);
     cudaError_t e = c.vin.ensure(n * sizeof(float));
     if (e != cudaSuccess) return fail_cuda(e, what);
-    fy::HostCopy copy(n * sizeof(float));
+    fy::HostCopy copy(n * sizeof(float), in, out);
     if ((e = copy.to_device(c.vin.p, in, n * sizeof(float), st)) != cudaSuccess) return fail_cuda(e, what);
     // dst aliases the device copy of src: P1 consumes src before P5 writes dst
     if ((rc = enqueue_deconv(c.vin.p, 0, 0.0, 0.0, c.vin.as<float>(), nx, nz, ny, nx, p, param, kind, fz2s, st,

@@ -1,6 +1,6 @@
 """The host deconvolutions on buffers that are not plain host memory. Under unified addressing the
-copies take device, managed and pinned addresses as well, below and above the size from which plain
-host memory is staged (1 MB); the bytes are the same, so the tolerance is none."""
+copies take device, managed and pinned addresses as well, below and above the sizes from which plain
+host memory is staged (4 MB); the bytes are the same, so the tolerance is none."""
 import ctypes as C
 
 import numpy as np
@@ -9,7 +9,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("shape", [(64, 64, 63), (64, 64, 64), (70, 128, 257)])
+@pytest.mark.parametrize("shape", [(64, 64, 63), (64, 64, 64), (90, 128, 257)])
 @pytest.mark.parametrize("src", ["host", "pinned", "device"])
 @pytest.mark.parametrize("dst", ["host", "pinned", "device"])
 def test_buffers(gpu, src, dst, shape):

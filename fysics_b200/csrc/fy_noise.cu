@@ -1402,11 +1402,14 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
     const int r = win / 2;
     const float inv_wc = (float)(1.0 / ((double)win * win * win));
     const unsigned g = grid_sel(n, sms), gc = grid_sel(Lay.cap, sms);
-    // passes that usually exit at once (the radix passes): one CTA per SM, four for the bins', so
-    // the common case schedules few empty CTAs; when they do run, their grid-stride loops cover
-    // every voxel
-    const unsigned gs = (unsigned)(g < (unsigned)sms ? g : (unsigned)sms);
-    const unsigned gs4 = (unsigned)(g < 4u * (unsigned)sms ? g : 4u * (unsigned)sms);
+    // Passes that usually exit at once (the radix passes): few and large CTAs, so the common case
+    // schedules few empty ones; when they do run, their grid-stride loops cover every voxel. What bounds
+    // them then is latency (means: two CTAs of 512 threads per SM 262 us a pass over 512^3, one of 256
+    // 436) and the CTAs' histograms joining the field's (bins of one value each, 512^3, four passes:
+    // one CTA of 1024 threads per SM 1410 us, four of 256 2000, four of 512 1999). In a batch, where every
+    // volume brings its CTAs, small ones exit faster: 16 cubes of 96..128 take 947 us so and 994 us
+    // with the large ones.
+    auto per_sm = [&](unsigned k) { return g < k * (unsigned)sms ? g : k * (unsigned)sms; };
     // candidate lists hold a few percent of the voxels (their capacity is n/8): two CTAs per SM
     const unsigned gcl = (unsigned)(gc < 2u * (unsigned)sms ? gc : 2u * (unsigned)sms);
     const size_t smem_hist = kHist * sizeof(unsigned int);
@@ -1432,7 +1435,10 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
     RUN(512, 1, k_mean_bucket, gcl, 512, smem_hist, ctl, cval, clab, lc_mean);
     RUN(256, 1, k_mean_collect, gcl, 256, 0, ctl, cval, clab, keys, lc_mean);
     RUN(kBoundThreads, 1, k_cand_select, 2, kBoundThreads, 3 * smem_stats, ctl, keys, lc_mean, (int)kMeanWin, (int)kMeanCand, 1);
-    for (int sh = 24; sh >= 0; sh -= 8) RUN(256, 1, k_mean_radix, gs, 256, smem_hist, mean, ctl, cval, clab, sh);
+    for (int sh = 24; sh >= 0; sh -= 8) {
+        if (L.record) RUN(256, 1, k_mean_radix, per_sm(1), 256, smem_hist, mean, ctl, cval, clab, sh);
+        else RUN(512, 1, k_mean_radix, per_sm(2), 512, smem_hist, mean, ctl, cval, clab, sh);
+    }
     if (!L.record) fy_prof_mark(st, "noise.lohi");
     // the per-bin flat_pct percentile of the variance, the same way. The sample lists use the
     // candidate region when it is large enough (the counting pass refills it afterwards).
@@ -1449,7 +1455,10 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
         RUN(256, 1, k_bin_collect, gcl, 256, 0, ctl, cval, clab, keys, lc_bin);
         RUN(kBoundThreads, 1, k_cand_select, NB, kBoundThreads, 3 * smem_stats, ctl, keys, lc_bin, (int)kBinWin, (int)kBinCand, 2);
     }
-    for (int sh = 24; sh >= 0; sh -= 8) RUN(256, 1, k_bin_radix, gs4, 256, smem_hist, mean, var, bin, ctl, cval, clab, sh);
+    for (int sh = 24; sh >= 0; sh -= 8) {
+        if (L.record) RUN(256, 1, k_bin_radix, per_sm(4), 256, smem_hist, mean, var, bin, ctl, cval, clab, sh);
+        else RUN(1024, 1, k_bin_radix, per_sm(1), 1024, smem_hist, mean, var, bin, ctl, cval, clab, sh);
+    }
     RUN(32, 1, k_noise_fit, 1, 32, 0, ctl);
     if (!L.record) fy_prof_mark(st, "noise.bin_select");
     return cudaSuccess;

@@ -687,6 +687,12 @@ extern "C" int fy_gpu_phase_correlate_batch(const float* d_fixed, const float* d
     } else {
         at_once = 1;
     }
+    // on every way out, errors among them: launches that use the workspace may be in flight
+    struct Release {
+        cudaStream_t st;
+        bool on;
+        ~Release() { if (on) fy::ws_release(st); }
+    } release{st, pws != ws};
     int launches = 0;
     for (int i = 0; i < npairs; i += at_once) {
         const int k = npairs - i < at_once ? npairs - i : at_once;
@@ -697,7 +703,6 @@ extern "C" int fy_gpu_phase_correlate_batch(const float* d_fixed, const float* d
                                    st)) != cudaSuccess)
             return fail_cuda(e, what);
     }
-    if (pws != ws) fy::ws_release(st);
     fy::count_launch(launches);
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail_cuda(e, what);
     for (int i = 0; i < npairs; ++i) {

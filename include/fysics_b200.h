@@ -395,7 +395,10 @@ int    fy_gpu_tune_value(const char *knob);
 
 /* Phase correlation of `npairs` device volume pairs (fixed[i], moving[i] at a stride of
  * nz*ny*nx floats) with fy_phase_correlate's semantics (fysics.h:311-313). d_scratch holds
- * fy_gpu_phase_correlate_scratch_bytes(). Results go to host arrays: shift[3*npairs],
+ * fy_gpu_phase_correlate_scratch_bytes(): the windows, and one pair's workspace. Where two or more
+ * pairs' workspaces fit 256 MB, that many are correlated at once in device memory of the calling
+ * thread (up to 256 MB and 6% slack, kept until fy_gpu_release; growing it frees the old block, which
+ * waits for the device); where it cannot be had, one by one in d_scratch. Results go to host arrays: shift[3*npairs],
  * peak[npairs] and peak_index[npairs] (nullable; flat index of the integer peak in the
  * power-of-two padded surface), status[npairs] (0 ok, 1 degenerate input). Synchronises
  * `stream` before returning. */

@@ -15,8 +15,9 @@
 // order statistics), so its output equals fy_gpu_restore_u8's bit for bit. The batched form
 // covers the chain with the noise model's eps and the shared noise/guided window without
 // rings or a radial model (the configuration of a batch of independent cubes); other
-// configurations, and volumes whose rows are not a multiple of 4 floats (no tensor-copy
-// staging), run one volume after another through fy_gpu_restore_u8.
+// configurations, and batches with a volume whose rows are not a multiple of 4 floats (the
+// deconvolved volumes' rows are dense here, so tensor copies could not stage them), run one
+// volume after another through fy_gpu_restore_u8.
 #include <string.h>
 
 #include <algorithm>
@@ -42,7 +43,8 @@ void fy_noise_batch_pack(const NoiseBatch* b, void* host);
 int fy_noise_batch_steps(const NoiseBatch* b);
 cudaError_t fy_noise_batch_launch(const NoiseBatch* b, const void* dev, cudaStream_t st);
 void fy_noise_batch_free(NoiseBatch* b);
-fyzb::Params fy_noise_stats_params(const float* in, int nz, int ny, int nx, int win, float* scratch, float* guided_mv);
+fyzb::Params fy_noise_stats_params(const float* in, int nz, int ny, int nx, int win, float* scratch, float* guided_mv,
+                                   int in_pitch);
 
 namespace {
 size_t al256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -182,12 +184,13 @@ extern "C" int fy_gpu_restore_u8_batch(const fy_batch_cube* cubes, int n, const 
         d.dpitch = q.nx;
         d.spec = c.bspec[i % K].as<float2>();
         float* mv = reinterpret_cast<float*>(A + off_mv[i]);
-        const fyzb::Params ps = fy_noise_stats_params(d.dst, q.nz, q.ny, q.nx, win, scr[i], mv);
+        const fyzb::Params ps = fy_noise_stats_params(d.dst, q.nz, q.ny, q.nx, win, scr[i], mv, d.dpitch);
         long long items = fyzb::make_job<fyzb::ZB_NOISE>(js[i], ps, win / 2, c.sms, total_s);
         if (items < 0) return fail(FY_ECUDA, "%s: volume %d: tensor map", what, i);
         total_s += items;
         fyzb::Params pg{};
         pg.nz = q.nz; pg.ny = q.ny; pg.nx = q.nx;
+        pg.pf0 = fy_pitch(q.nx); pg.pg = d.dpitch;
         pg.f0 = mv; pg.guide = d.dst; pg.o0 = q.out; pg.out_mode = 0; pg.eps = 0.f;
         pg.eps_ptr = fy_noise_eps_ptr(ctlp[i]);
         items = fyzb::make_job<fyzb::ZB_GUIDED_OUT_MV>(jg[i], pg, radius, c.sms, total_g);

@@ -1131,24 +1131,6 @@ FY_D void k_bwin_count(const float* __restrict__ mean, const float* __restrict__
     }
 }
 
-FY_D void sort_small(double* v, int n) {
-    for (int i = 1; i < n; ++i) {
-        const double k = v[i];
-        int j = i - 1;
-        while (j >= 0 && v[j] > k) { v[j + 1] = v[j]; --j; }
-        v[j + 1] = k;
-    }
-}
-FY_D double pct_small(double* v, int n, double pct) {       // percentile() on <= 24 values
-    if (n <= 0) return 0.0;
-    sort_small(v, n);
-    const double idx = pct / 100.0 * (n - 1);
-    const int lo = (int)idx;
-    const double f = idx - lo;
-    if (lo + 1 < n) return v[lo] * (1 - f) + v[lo + 1] * f;
-    return v[lo];
-}
-
 // IRLS fit (FP64) and outputs. One warp: lane b handles bin b, so the bins' loads are in flight
 // together. The used bins are compacted in bin order; the weights, residuals and the median of the
 // residuals are formed by one lane per bin, the five weighted sums by lane 0 in the reference's
@@ -1301,6 +1283,21 @@ unsigned long long weyl_step(unsigned long long n) {
 
 size_t fy_noise_scratch_floats(size_t n) { return noise_layout(n).total; }
 
+// The statistics pass's parameters for one volume, rows of `in` in_pitch floats apart (0: nx): mean and
+// variance fields dense in the scratch, the guided (mean, var) pairs (optional) in rows of fy_pitch(nx).
+fyzb::Params fy_noise_stats_params(const float* in, int nz, int ny, int nx, int win, float* scratch, float* guided_mv,
+                                   int in_pitch) {
+    const NoiseLayout Lay = noise_layout((size_t)nz * ny * nx);
+    fyzb::Params sp{};
+    sp.nz = nz; sp.ny = ny; sp.nx = nx;
+    sp.f0 = in; sp.o0 = scratch + Lay.mean; sp.o1 = scratch + Lay.var; sp.o2 = guided_mv;
+    sp.inv_wc = (float)(1.0 / ((double)win * win * win));
+    sp.wci = win * win * win;
+    sp.pf0 = in_pitch;
+    sp.pmv = fy_pitch(nx);
+    return sp;
+}
+
 namespace {
 
 // ---------------------------------------------------------------- launching: one cube or a batch
@@ -1399,8 +1396,6 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
     uint32_t* keys = (uint32_t*)(scratch + Lay.bin);
     float* cval = scratch + Lay.cval;
     uint8_t* clab = (uint8_t*)(scratch + Lay.clab);
-    const int r = win / 2;
-    const float inv_wc = (float)(1.0 / ((double)win * win * win));
     const unsigned g = grid_sel(n, sms), gc = grid_sel(Lay.cap, sms);
     // Passes that usually exit at once (the radix passes): few and large CTAs, so the common case
     // schedules few empty ones; when they do run, their grid-stride loops cover every voxel. What bounds
@@ -1418,12 +1413,8 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
     const long long lc_mean = n / 8 < kListMax ? n / 8 : kListMax, lc_bin = n / (4 * NB) < kListMax ? n / (4 * NB) : kListMax;
     const size_t smem_stats = 2048 * sizeof(unsigned int);
     if (stats) {   // 1. stats
-        fyzb::Params sp{};
-        sp.nz = nz; sp.ny = ny; sp.nx = nx;
-        sp.f0 = in; sp.o0 = mean; sp.o1 = var; sp.o2 = guided_mv;
-        sp.inv_wc = inv_wc; sp.wci = win * win * win;
-        sp.pf0 = in_pitch; sp.pmv = fy_pitch(nx);
-        cudaError_t e0 = fyzb::launch<fyzb::ZB_NOISE>(sp, r, sms, st);
+        cudaError_t e0 = fyzb::launch<fyzb::ZB_NOISE>(fy_noise_stats_params(in, nz, ny, nx, win, scratch, guided_mv, in_pitch),
+                                                      win / 2, sms, st);
         if (e0 != cudaSuccess) return e0;
         ++launches;
         if (!L.record) fy_prof_mark(st, "noise.stats");
@@ -1559,18 +1550,6 @@ cudaError_t fy_noise_batch_launch(const NoiseBatch* b, const void* dev, cudaStre
     return cudaSuccess;
 }
 void fy_noise_batch_free(NoiseBatch* b) { delete b; }
-// The statistics pass's parameters for one volume (box pass ZB_NOISE writing the guided
-// (mean, var) pairs too), as noise_sequence forms them.
-fyzb::Params fy_noise_stats_params(const float* in, int nz, int ny, int nx, int win, float* scratch, float* guided_mv) {
-    const NoiseLayout Lay = noise_layout((size_t)nz * ny * nx);
-    fyzb::Params sp{};
-    sp.nz = nz; sp.ny = ny; sp.nx = nx;
-    sp.f0 = in; sp.o0 = scratch + Lay.mean; sp.o1 = scratch + Lay.var; sp.o2 = guided_mv;
-    sp.inv_wc = (float)(1.0 / ((double)win * win * win));
-    sp.wci = win * win * win;
-    return sp;
-}
-
 // Copy the model out of a finished control block (device -> host, async on st).
 cudaError_t fy_noise_read(const void* ctl_mem, double* g, double* b, double* noise_ref, double* ref_intensity,
                           int* used, cudaStream_t st) {

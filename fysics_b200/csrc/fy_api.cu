@@ -338,6 +338,7 @@ int enqueue_deconv(const void* src, int src_u8, double fmin, double fmax, float*
     if ((rc = deconv_tables(d.g, p, param, kind, fz2s, st, d))) return rc;
     d.src = src; d.src_u8 = src_u8; d.dst = dst; d.dpitch = dpitch;
     dewindow_params(fmin, fmax, d.lo, d.scale);
+    d.sms = c.sms;
     if ((e = fy_launch_deconv(d, st)) != cudaSuccess) return fail_cuda(e, what);
     fy::count_launch(5);
     return FY_OK;
@@ -394,6 +395,7 @@ int fy_deconv_setup(int nz, int ny, int nx, const fy_physics* p, double& param, 
     d.twx = fy::twiddles(d.g.px); d.twy = fy::twiddles(d.g.py); d.twz = fy::twiddles(d.g.pz);
     if (!d.twx || !d.twy || !d.twz) return fail(FY_ENOMEM, "%s: twiddle tables", what);
     dewindow_params(fmin, fmax, d.lo, d.scale);
+    d.sms = ctx().sms;
     return FY_OK;
 }
 

@@ -23,6 +23,7 @@ struct DeconvLaunch {
     const float* lut;         // FY_LUT_N+1 floats
     const double *fz2, *fy2, *fx2;
     double us;                // LUT index scale FY_LUT_N / umax
+    int sms;                  // SMs of the device (the column passes' tiles)
 };
 cudaError_t fy_launch_deconv(const DeconvLaunch& d, cudaStream_t st);
 // Compile-time-plan pass `pass` (1..5) for axis length n; cudaErrorNotSupported when n has no

@@ -345,9 +345,9 @@ inline cudaError_t launch(K k, unsigned grid, int nt, size_t smem, cudaStream_t 
 // stored; sign +1: rows < keep_rows stored.
 template <int N>
 inline cudaError_t launch_y(float2* spec, const SpecGeom& g, const float2* tw, int nplanes, int sign, int keep_rows,
-                            cudaStream_t st) {
+                            int sms, cudaStream_t st) {
     using C = Col<N>;
-    const ColTiles ct = col_tiles(g.hx, nplanes, C::W, N <= 256 ? 2 * 148L * C::minb : LONG_MAX);
+    const ColTiles ct = col_tiles(g.hx, nplanes, C::W, N <= 256 ? 2L * sms * C::minb : LONG_MAX);
     if (sign > 0) return launch(k_col_y<N, 1, false>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, keep_rows);
     if (g.ny == N) return launch(k_col_y<N, -1, false>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, N, N);
     return launch(k_col_y<N, -1, true>, ct.total, C::NT, C::smem, st, spec, g, ct, tw, g.ny, N);
@@ -369,11 +369,11 @@ cudaError_t deconv_pass(int pass, const DeconvLaunch& d, cudaStream_t st) {
         return pad ? FY_ROW_FWD(float, true) : FY_ROW_FWD(float, false);
 #undef FY_ROW_FWD
     }
-    case 2: return launch_y<N>(d.spec, g, d.twy, g.nz, -1, g.py, st);
-    case 4: return launch_y<N>(d.spec, g, d.twy, g.nz, +1, g.ny, st);
+    case 2: return launch_y<N>(d.spec, g, d.twy, g.nz, -1, g.py, d.sms, st);
+    case 4: return launch_y<N>(d.spec, g, d.twy, g.nz, +1, g.ny, d.sms, st);
     case 3: {
         using C = Col<N>;
-        const ColTiles ct = col_tiles(g.hx, g.py, C::W, 148L * C::minb);
+        const ColTiles ct = col_tiles(g.hx, g.py, C::W, (long)d.sms * C::minb);
         if (g.nz == N)
             return launch(k_col_z<N, false>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);
         return launch(k_col_z<N, true>, ct.total, C::NT, C::smem, st, d.spec, g, ct, d.twz, d.lut, d.fz2, d.fy2, d.fx2, d.us);

@@ -417,7 +417,8 @@ static_assert(kSampleMax <= kBoundThreads * kKeysPerThread && kBinListMax <= kBo
               kListMax <= kBoundThreads * kKeysPerThread, "every list fits the block's registers");
 constexpr double kWinSigmas = 5.0;
 // Test hook: bit 0 forces the mean percentiles, bit 1 the bins, to the radix passes over the
-// whole field; noise_window_used records (bits 0/1) which windows produced their result.
+// whole field, bits 2 and 3 to those over the windows' candidates; noise_window_used records (bits
+// 0/1) which windows produced their result and (bits 2/3) which of them by the candidates' passes.
 static __device__ int noise_force_radix;
 static __device__ int noise_window_used;
 
@@ -742,13 +743,13 @@ FY_D void for_each_cand(const NoiseCtl* __restrict__ ctl, const float* __restric
 
 // Bucket step for nt targets of nb buckets: the candidates' histogram; the last CTA finds per target the buckets
 // of r = k - below and r + 1. `field` and `cand`: the modes of the radix passes that take over;
-// lcap: keys that a target can collect.
+// force_bit: the test hook's bit for the latter; lcap: keys that a target can collect.
 FY_D void cand_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab, int nt,
-                      int nb, long long lcap, int field, int cand) {
+                      int nb, long long lcap, int field, int cand, int force_bit) {
     extern __shared__ unsigned int rh[];
     __shared__ float sv0[NB], svs[NB];
     __shared__ int s_field, s_cand;
-    const int t = threadIdx.x, lane = t & 31;
+    const int t = threadIdx.x, lane = t & 31, forced = noise_force_radix & force_bit;
     const unsigned full = 0xffffffffu;
     for (int i = t; i < nt * nb; i += blockDim.x) rh[i] = 0;
     if (t < nt) { sv0[t] = ctl->cv0[t]; svs[t] = ctl->cvs[t]; }
@@ -790,7 +791,7 @@ FY_D void cand_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval
             ctl->cb1[g] = b1;
             ctl->crank[g] = r - (long long)before;
             ctl->trank[g] = r;                            // for the radix passes over the candidates
-            if (cnt > lcap) s_cand = 1;
+            if (cnt > lcap || forced) s_cand = 1;
         }
     }
     __syncthreads();
@@ -849,7 +850,7 @@ FY_D void k_cand_select(NoiseCtl* __restrict__ ctl, const uint32_t* __restrict__
     fy_pdl_wait();
     extern __shared__ unsigned int wsh[];                // 3 * 2048 counters
     const int g = vbx(), t = threadIdx.x, mode = ctl->mode;
-    if (t == 0 && g == 0 && (mode == win || mode == cand)) atomicOr(&noise_window_used, used_bit);
+    if (t == 0 && g == 0 && (mode == win || mode == cand)) atomicOr(&noise_window_used, mode == cand ? used_bit * 5 : used_bit);
     if (mode != win || g >= ctl->ntarget || !ctl->tactive[g]) return;
     const int c = (int)ctl->ccnt[g], r = (int)ctl->crank[g];
     const bool has_next = ctl->tk[g] + 1 < ctl->tgroup_n[g];
@@ -871,7 +872,7 @@ FY_D void k_cand_select(NoiseCtl* __restrict__ ctl, const uint32_t* __restrict__
 FY_D void k_mean_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
                         long long lcap) {
     fy_pdl_wait();
-    if (ctl->mode == kMeanWin) cand_bucket(ctl, cval, clab, 2, kMeanBuckets, lcap, kMeanField, kMeanCand);
+    if (ctl->mode == kMeanWin) cand_bucket(ctl, cval, clab, 2, kMeanBuckets, lcap, kMeanField, kMeanCand, 4);
 }
 FY_D void k_mean_collect(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
                          uint32_t* __restrict__ list, long long lcap) {
@@ -881,7 +882,7 @@ FY_D void k_mean_collect(NoiseCtl* __restrict__ ctl, const float* __restrict__ c
 FY_D void k_bin_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
                        long long lcap) {
     fy_pdl_wait();
-    if (ctl->mode == kBinWin) cand_bucket(ctl, cval, clab, NB, kBinBuckets, lcap, kBinField, kBinCand);
+    if (ctl->mode == kBinWin) cand_bucket(ctl, cval, clab, NB, kBinBuckets, lcap, kBinField, kBinCand, 8);
 }
 FY_D void k_bin_collect(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval, const uint8_t* __restrict__ clab,
                         uint32_t* __restrict__ list, long long lcap) {

@@ -259,9 +259,10 @@ int fy_gpu_test_box_first_wait(int polls);
  * 99th percentiles of the local means and the per-bin percentiles of the local variances
  * come from sample-guided key windows over one pass each, with exact radix passes over the
  * whole field when a window misses. force_radix bit 0 sends the means, bit 1 the bins, to
- * the radix passes every time (0 restores the windows). *window_used (optional) receives
- * which windows produced their result (bit 0 means, bit 1 bins) since the previous call.
- * Both paths give the same exact order statistics. Synchronises the device. */
+ * the radix passes every time, bits 2 and 3 to radix passes over the windows' candidates, which
+ * otherwise run when too many of these are equal (0 restores the windows). *window_used
+ * (optional) receives which windows produced their result (bit 0 means, bit 1 bins), and which of
+ * them by the candidates' passes (bits 2 and 3), since the previous call. All paths give the same exact order statistics. Synchronises the device. */
 int fy_gpu_test_noise_paths(int force_radix, int *window_used);
 
 /* Device-pointer forms of the drop-in calls, enqueued on `stream` (a cudaStream_t, NULL =

@@ -749,7 +749,7 @@ FY_D void cand_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval
     extern __shared__ unsigned int rh[];
     __shared__ float sv0[NB], svs[NB];
     __shared__ int s_field, s_cand;
-    const int t = threadIdx.x, lane = t & 31, forced = noise_force_radix & force_bit;
+    const int t = threadIdx.x, lane = t & 31;
     const unsigned full = 0xffffffffu;
     for (int i = t; i < nt * nb; i += blockDim.x) rh[i] = 0;
     if (t < nt) { sv0[t] = ctl->cv0[t]; svs[t] = ctl->cvs[t]; }
@@ -762,6 +762,7 @@ FY_D void cand_bucket(NoiseCtl* __restrict__ ctl, const float* __restrict__ cval
     for (int i = t; i < nt * nb; i += blockDim.x)
         if (rh[i]) atomicAdd(&ctl->hist[i], rh[i]);
     if (!last_cta(ctl)) return;
+    const int forced = noise_force_radix & force_bit;
 #pragma unroll 4
     for (int i = t; i < nt * nb; i += blockDim.x) {
         rh[i] = __ldcg(&ctl->hist[i]);
@@ -1405,7 +1406,10 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
     // one CTA of 1024 threads per SM 1410 us, four of 256 2000, four of 512 1999). In a batch, where every
     // volume brings its CTAs, small ones exit faster: 16 cubes of 96..128 take 947 us so and 994 us
     // with the large ones.
-    auto per_sm = [&](unsigned k) { return g < k * (unsigned)sms ? g : k * (unsigned)sms; };
+    auto per_sm = [&](unsigned k, unsigned threads) {     // k CTAs per SM, fewer where a step covers the field
+        const unsigned steps = (g * 256 + threads - 1) / threads;
+        return steps < k * (unsigned)sms ? steps : k * (unsigned)sms;
+    };
     // candidate lists hold a few percent of the voxels (their capacity is n/8): two CTAs per SM
     const unsigned gcl = (unsigned)(gc < 2u * (unsigned)sms ? gc : 2u * (unsigned)sms);
     const size_t smem_hist = kHist * sizeof(unsigned int);
@@ -1428,8 +1432,8 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
     RUN(256, 1, k_mean_collect, gcl, 256, 0, ctl, cval, clab, keys, lc_mean);
     RUN(kBoundThreads, 1, k_cand_select, 2, kBoundThreads, 3 * smem_stats, ctl, keys, lc_mean, (int)kMeanWin, (int)kMeanCand, 1);
     for (int sh = 24; sh >= 0; sh -= 8) {
-        if (L.record) RUN(256, 1, k_mean_radix, per_sm(1), 256, smem_hist, mean, ctl, cval, clab, sh);
-        else RUN(512, 1, k_mean_radix, per_sm(2), 512, smem_hist, mean, ctl, cval, clab, sh);
+        if (L.record) RUN(256, 1, k_mean_radix, per_sm(1, 256), 256, smem_hist, mean, ctl, cval, clab, sh);
+        else RUN(512, 1, k_mean_radix, per_sm(2, 512), 512, smem_hist, mean, ctl, cval, clab, sh);
     }
     if (!L.record) fy_prof_mark(st, "noise.lohi");
     // the per-bin flat_pct percentile of the variance, the same way. The sample lists use the
@@ -1448,8 +1452,8 @@ cudaError_t noise_sequence(NoiseLaunch& L, const float* in, int nz, int ny, int 
         RUN(kBoundThreads, 1, k_cand_select, NB, kBoundThreads, 3 * smem_stats, ctl, keys, lc_bin, (int)kBinWin, (int)kBinCand, 2);
     }
     for (int sh = 24; sh >= 0; sh -= 8) {
-        if (L.record) RUN(256, 1, k_bin_radix, per_sm(4), 256, smem_hist, mean, var, bin, ctl, cval, clab, sh);
-        else RUN(1024, 1, k_bin_radix, per_sm(1), 1024, smem_hist, mean, var, bin, ctl, cval, clab, sh);
+        if (L.record) RUN(256, 1, k_bin_radix, per_sm(4, 256), 256, smem_hist, mean, var, bin, ctl, cval, clab, sh);
+        else RUN(1024, 1, k_bin_radix, per_sm(1, 1024), 1024, smem_hist, mean, var, bin, ctl, cval, clab, sh);
     }
     RUN(32, 1, k_noise_fit, 1, 32, 0, ctl);
     if (!L.record) fy_prof_mark(st, "noise.bin_select");

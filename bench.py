@@ -162,14 +162,13 @@ def algorithmic_bytes(name: str, n: int, geo: dict) -> float | None:
 TIMED_MARKS = "noise,guided"
 
 # DRAM bytes per voxel of each instrumented span: dram__bytes_read.sum + dram__bytes_write.sum
-# of its kernel's launch in an ncu capture of this chain on a 384^3 cube (one kernel per
-# capture, on the smaller cube; every span's traffic grows with the voxel count), divided by
-# its voxels. The two selection spans give their counting pass only: their other launches
-# run over candidate lists of a few percent of the voxels.
+# of its kernel's launch in an ncu capture of this chain on a 384^3 cube (every span's traffic
+# grows with the voxel count), divided by its voxels. The two selection spans give their counting
+# pass only: their other launches run over candidate lists of a few percent of the voxels.
 DRAM_BYTES_PER_VOXEL = {
-    "deconv.x_fwd": 4.087, "deconv.y_fwd": 7.599, "deconv.z_weight": 8.198, "deconv.y_inv": 7.602,
-    "deconv.x_inv": 7.539, "noise.stats": 19.142, "noise.lohi": 4.108, "noise.bin_select": 8.227,
-    "guided": 15.954,
+    "deconv.x_fwd": 4.103, "deconv.y_fwd": 7.368, "deconv.z_weight": 7.357, "deconv.y_inv": 7.361,
+    "deconv.x_inv": 7.421, "noise.stats": 19.107, "noise.lohi": 4.053, "noise.bin_select": 8.149,
+    "guided": 15.937,
 }
 
 

@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(KB<E>::nt, 2) k_x_fwd(const T* __restrict__ sr
 // ---------------------------------------------------------------- P2
 // CTA = (column tile of W half-spectrum columns, stored plane z). Pass-0 inputs come
 // straight from global memory (W consecutive columns = one 8W-byte run per point);
-// rows >= ny are the reflected (or zero) rows.
+// rows >= ny are the reflected rows.
 template <int N, int E>
 __global__ void __launch_bounds__(KB<E>::nt, 2) k_y_fwd(float2* __restrict__ spec, SpecGeom g, const __grid_constant__ FftPlan pl,
                                                  const float2* __restrict__ tw, int wlog) {

@@ -98,7 +98,7 @@ size_t fy_guided_fused_scratch_floats(int nz, int ny, int nx) { return 2 * round
 
 // Exact guided filter for r in [1, 4] as two z-sliding box passes (fy_zbox.cuh):
 // in -> interleaved (a, b) pairs into ab_ws, then box(a), box(b) -> out. ab_ws holds
-// fy_guided_fused_scratch_floats(n) floats; out may alias in. mode 1 writes box(a) to out
+// fy_guided_fused_scratch_floats(nz, ny, nx) floats; out may alias in. mode 1 writes box(a) to out
 // and box(b) to out_b instead of the filtered volume. The pairs' rows are fy_pitch(nx) voxels apart, so
 // the second pass stages them by TMA whatever nx is.
 cudaError_t fy_launch_guided_fused(const float* in, float* out, float* out_b, float* ab_ws, int nz, int ny, int nx,

@@ -13,8 +13,8 @@
 //      sample-guided windows (section 2w): sample and bounds, count, bucket, collect. Radix passes
 //      over the window's candidates or over the whole field stand behind them (section 2r) and
 //      exit at once when the windows gave the answer.
-//   3. k_noise_fit: one thread, FP64: IRLS line fit var = g*I + b (noise.c:137-172) and
-//      noise_ref = sqrt(max(g*ref + b, ..))*1.15 (noise.c:181-187), plus the guided eps
+//   3. k_noise_fit: one warp, FP64 (five lanes form the weighted sums): IRLS line fit
+//      var = g*I + b (noise.c:137-172) and noise_ref = sqrt(max(g*ref + b, ..))*1.15 (noise.c:181-187), plus the guided eps
 //      (3*noise_ref)^2 floored at 1e-8 (noise.c:197-202).
 // The launch sequence is fixed (no host decisions), so a chain can keep it on one stream.
 #include <cuda/std/tuple>

@@ -36,7 +36,7 @@ constexpr int head_r0(int n) { return n % 3 ? (n <= 128 ? 4 : 8) : 3; }
 constexpr int head_r1(int n) { return n % 3 ? 4 : 8; }
 constexpr int tpl(int n) { return n / elems(n); }
 
-// exp(2*pi*i*m/64) and exp(2*pi*i*m/24), FP64 rounded once to float like the twiddle tables.
+// exp(2*pi*i*m/32) and exp(2*pi*i*m/24), FP64 rounded once to float like the twiddle tables.
 template <int PA> constexpr float root_c(int m) {
     constexpr float c32[32] = {
         0x1.0000000000000p+0f, 0x1.f6297c0000000p-1f, 0x1.d906bc0000000p-1f, 0x1.a9b6620000000p-1f, 0x1.6a09e60000000p-1f,

@@ -12,11 +12,12 @@ namespace rf {
 // column index fastest. Its tile crosses shared memory once per transform, stored point-major
 // (s[i*W + l]: a half warp's 16 columns are 16 consecutive float2, no conflicts).
 // What bounds them: HBM at 512 (the Y passes move 1.07 GB in 180 us, 0.91 of the measured copy
-// rate), latency below. Sixteen warps an SM with 128 registers and no spills: at 512^3 the Z pass
-// takes 307 us so, 379 us with 8-column tiles (64-byte runs) and 20 warps, 434 us with 24 warps at
-// 80 registers (spills, and more tiles in flight than HBM serves well). The shared-memory passes
-// that these replace took 237 (Y forward), 424 (Z) and 203 us (Y inverse) there; at 256^3 33, 57
-// and 27 us against 27, 37 and 23 now.
+// rate), latency below. Sixteen warps an SM with 128 registers (16 bytes of spills at most): at 512^3
+// the Z pass takes 313 us so; with its weight's position in 32 fraction bits it took 307, and in that
+// form 379 us with 8-column tiles (64-byte runs) and 20 warps, 434 us with 24 warps at 80 registers
+// (spills, and more tiles in flight than HBM serves well). The shared-memory passes that these replace
+// took 237 (Y forward), 424 (Z) and 203 us (Y inverse) there; at 256^3 33, 57 and 27 us against 25, 37
+// and 23 now.
 template <int N> struct Col {
     static constexpr int W = 16, NT = W * tpl(N);
     static constexpr int warps = elems(N) <= 24 ? 24 : 16;
@@ -32,9 +33,12 @@ template <int N> struct Col {
 // They take several times a regular tile's time (16 sectors a request), so they are made only where
 // at least `least` regular tiles hide them; below that the partly filled tiles are faster. Measured
 // (us, shared against own): Y at 16 x 384^2 26.8 / 10.3, 16 x 512^2 22.5 / 12.3, 64^3 8.2 / 6.3, 192^3
-// 16.4 / 13.3, 256^3 26.6 / 28.6, 384^3 112.6 / 107, 512^3 190 / 179; Z at 128^3 14.3 / 12.3, 192^3
-// 20.5 / 22.5, 256^3 36.9 / 38.9, 384^3 186 / 201, 512^3 305 / 311. So a Y pass shares them from two
-// waves of CTAs on up to 256 points (above, a tile of its own is under 5% more work), a Z pass from one.
+// 16.4 / 13.3, 256^3 26.6 / 28.6, 384^3 113 / 107, 512^3 190 / 179; Z at 128^3 14.3 / 12.3, 192^3
+// 20.5 / 22.5, 256^3 36.9 / 38.9, 384^3 186 / 201, 512^3 305 / 311 (events around each pass). So a Y pass
+// shares them from two waves of CTAs on up to 256 points (above, a tile of its own is under 5% more
+// work), a Z pass from one. Phase correlation's passes always share (least = 0): of whole correlations,
+// shared against own, single pairs of few rows lose (8 x 512^2 107 / 96 us, 64^3 67 / 61) and many rows or
+// pairs gain (200^3 x 2 563 / 585, 64 pairs of 4 x 64^2 77 / 83).
 struct ColTiles {
     int regular;              // tiles per row over the kx < px/2 columns (or over all hx columns)
     int rows;                 // rows (planes of a Y pass, y of a Z pass)
